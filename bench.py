@@ -127,7 +127,7 @@ def level0_kernel_bytes(w):
 
 def kernels_per_frame(w, tuning: str) -> int:
     """Kernel launches of one frame: the pyramid (levels 1 and 2 in one launch, each deeper
-    level one more), then per level one fused kernel (streaming or tile) or the per-stage
+    level one more), then per level one fused kernel (streaming, tile or slab) or the per-stage
     kernels (model, 2N propagation passes, update, 2S smoothing passes)."""
     L = w["levels"]
     parts = [p.strip() for p in tuning.split(";")]
@@ -140,7 +140,7 @@ def kernels_per_frame(w, tuning: str) -> int:
         m = w["maxflow"] / (2 ** min(l, L - 1))
         N = int(np.ceil(np.float32(m)))
         S = w["smooth"][l]
-        fused = l < len(parts) and ("fused" in parts[l] or "tile" in parts[l])
+        fused = l < len(parts) and any(k in parts[l] for k in ("fused", "tile", "slab"))
         n += 1 if fused else 2 + 2 * N + 2 * S
     return n
 

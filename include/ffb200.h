@@ -128,9 +128,9 @@ ff_status ff_filter_get_propagation_border(const ff_filter* f, int* border);
 ff_status ff_filter_get_propagation_iterations(const ff_filter* f, int level, int* iterations);
 
 /* Kernel selection per level: 0 per-stage kernels, 1 the streaming fused per-level kernel
- * wherever it is instantiated, 2 automatic (default: the autotuned choice, else the
- * streaming kernel for levels of at least 200,000 pixels and the tile-fused kernel below),
- * 3 the tile-fused kernel wherever it fits in shared memory.  All modes give bit-identical
+ * wherever it is instantiated, 2 automatic (default: the autotuned choice, else by
+ * size and smoothing the slab kernel, the streaming kernel for the largest levels or the
+ * tile-fused kernel for the smallest delta levels), 3 the tile-fused kernel wherever it fits in shared memory.  All modes give bit-identical
  * results. */
 ff_status ff_filter_set_fused(ff_filter* f, int mode);
 
@@ -138,8 +138,8 @@ ff_status ff_filter_set_fused(ff_filter* f, int mode);
  * use and re-captured after any parameter change).  Off by default. */
 ff_status ff_filter_set_graphs(ff_filter* f, int enabled);
 /* Autotuner: on the current inputs, time each level's per-stage kernels, its streaming
- * fused kernel at several band heights and its tile-fused kernel at several tile shapes
- * (`repetitions` runs each); then, for pyramids, time whole frames over combinations of each
+ * fused kernel at several band heights, its slab kernel and its tile-fused kernel at several
+ * tile shapes (`repetitions` runs each); then, for pyramids, time whole frames over combinations of each
  * level's best choices (the levels share the GPU within a frame) from a snapshot of the state
  * that is restored afterwards, and keep the fastest combination, used while the mode is 2.
  * Needs one computed frame; results are unchanged because every candidate writes
@@ -150,7 +150,7 @@ ff_status ff_filter_autotune(ff_filter* f, int repetitions);
  * in a measurement that flushes L2 between frames. */
 ff_status ff_filter_autotune_flush(ff_filter* f, int repetitions, void* flush, size_t flush_bytes);
 /* Read or set one level's kernel choice (path: -1 untuned, 0 per-stage, 1 streaming fused,
- * 2 tile-fused; band: rows of a streaming band or the tile-shape index, 0 automatic), e.g.
+ * 2 tile-fused, 3 slab; band: rows of a streaming band or a slab or the tile-shape index, 0 automatic), e.g.
  * to reuse a saved autotuning result. */
 ff_status ff_filter_get_level_tuning(const ff_filter* f, int level, int* path, int* band);
 ff_status ff_filter_set_level_tuning(ff_filter* f, int level, int path, int band);

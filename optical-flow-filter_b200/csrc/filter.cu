@@ -602,6 +602,22 @@ bool Filter::tile_ok(int l, int cfg) const {
     return tile_available(v.delta, v.iters, v.smooth, v.W, v.H, cfg);
 }
 
+// can the slab kernel run this level?  It loads uint8 image rows as aligned 4-byte words (up
+// to the next multiple of 4 columns), everything else at its own alignment.
+bool Filter::slab_ok(int l) const {
+    const Level& v = lv_[l];
+    const uintptr_t ib = (uintptr_t)v.img;
+    const bool img_ok = ib % 4 == 0 && v.img_pitch % 4 == 0 && (v.item == 4 || v.img_owned || v.W % 4 == 0);
+    if (v.delta) {
+        const void* cpp = nullptr;
+        size_t cpitch = 0;
+        int chh = 0, cww = 0;
+        coarse_of(l, &cpp, &cpitch, &chh, &cww);
+        if (!cpp || (uintptr_t)cpp % 8 != 0 || cpitch % 8 != 0) return false;
+    }
+    return img_ok && slab_available(v.delta, v.iters, v.smooth);
+}
+
 LevelArgs Filter::level_args(int l) const {
     const Level& v = lv_[l];
     const int nxt = cur_ ^ 1;
@@ -646,18 +662,31 @@ void Filter::launch_fused(int l, int band, cudaStream_t s) {
     check_cuda(launch_fused_level(v.delta, v.iters, v.smooth, a, s), "fused level");
 }
 
+// In a pyramid frame the top level's tile or slab kernel is followed on the same stream by
+// level L-2's, which reads the top's output only from its update on: the top lets it start at
+// once, and it waits only before its update (so its propagation overlaps the top level).
+void Filter::chain_pdl(int l, LevelArgs& a) const {
+    if (kind_ != Kind::Pyramidal || L_ < 2 || !pdl_chain_) return;
+    auto chained = [&](int m) {
+        const int p = path_of(m, nullptr);
+        return p == kTile || p == kSlab;
+    };
+    if (l == L_ - 1 && chained(L_ - 2)) a.pdl_early_trigger = 1;
+    if (l == L_ - 2 && chained(L_ - 1)) a.pdl_late_wait = 1;
+}
+
+void Filter::launch_slab(int l, int rows, cudaStream_t s) {
+    const Level& v = lv_[l];
+    LevelArgs a = level_args(l);
+    a.band = rows;
+    chain_pdl(l, a);
+    check_cuda(launch_slab_level(v.delta, v.iters, v.smooth, a, s), "slab level");
+}
+
 void Filter::launch_tile(int l, int cfg, cudaStream_t s) {
     const Level& v = lv_[l];
     LevelArgs a = level_args(l);
-    // In a pyramid frame the top level's tile kernel is followed on the same stream by level
-    // L-2's, which reads the top's output only from its update on: the top lets it start at
-    // once, and it waits only before its update (so its propagation overlaps the top level).
-    if (kind_ == Kind::Pyramidal && L_ >= 2 && pdl_chain_) {
-        int p_top = 0, p_next = 0;
-        const bool top_tile = path_of(L_ - 1, &p_top) == kTile, next_tile = path_of(L_ - 2, &p_next) == kTile;
-        if (l == L_ - 1 && next_tile) a.pdl_early_trigger = 1;
-        if (l == L_ - 2 && top_tile) a.pdl_late_wait = 1;
-    }
+    chain_pdl(l, a);
     if (fuse_pyramid_ && l == L_ - 1) {
         const Level& fine = lv_[0];
         a.pyr_src = fine.img;
@@ -682,11 +711,12 @@ void Filter::step_level(int l, cudaStream_t s) {
     switch (path_of(l, &param)) {
         case kStream: launch_fused(l, param, s); break;
         case kTile: launch_tile(l, param, s); break;
+        case kSlab: launch_slab(l, param, s); break;
         default: step_level_unfused(l, s);
     }
 }
 
-// the path a level step takes now; *param = band rows (streaming) or tile shape (tile)
+// the path a level step takes now; *param = band rows (streaming), slab rows or tile shape
 int Filter::path_of(int l, int* param) const {
     const Level& v = lv_[l];
     int dummy = 0;
@@ -708,14 +738,24 @@ int Filter::path_of(int l, int* param) const {
         p = v.tuned_band;
         return kTile;
     }
+    if (v.tuned_path == kSlab && slab_ok(l)) {
+        p = v.tuned_band;
+        return kSlab;
+    }
     if (v.tuned_path == kPerStage) return kPerStage;
-    // untuned: the streaming kernel keeps large levels in one pass over HBM; below
-    // kFusedMinPixels its warps are few and latency-bound, and the tile kernel spreads
-    // each stage over whole CTAs instead
-    if ((long)v.H * v.W >= kFusedMinPixels && fused_ok(l)) {
+    // Untuned.  The slab kernel's rows stay in shared memory, so it holds 2048x1088 in 2-3 waves;
+    // the streaming kernel passes over HBM once at any size, but its chain of stages per row
+    // grows with S.  Measured alone (us, slab / streaming / tile), delta levels: 160x120 N 4 S 2
+    // 18.0 / 54.7 / 15.9, 320x240 20.0 / 53.2 / 19.9, 640x480 26.1 / 58.9 / 34.3, 1280x720
+    // 45.3 / 62.9 / 69.4, 2048x1088 98.3 / 89.0 / 153.2 and with S 4 120.6 / 178.2 / 223.5; top
+    // levels: 160x120 N 2 S 2 11.8 / 28.1 / 11.7, 1280x720 26.1 / 38.4 / 40.3, 2048x1088
+    // 48.8 / 50.0 / 80.8 and with S 1 43.7 / 36.7 / 69.7.
+    const long px = (long)v.H * v.W;
+    if (px >= kStreamMinPixels && v.smooth <= (v.delta ? 2 : 1) && fused_ok(l)) {
         p = band_;
         return kStream;
     }
+    if ((!v.delta || px >= kSlabMinPixels) && slab_ok(l)) return kSlab;
     if (tile_ok(l, 0)) return kTile;
     return kPerStage;
 }
@@ -788,6 +828,7 @@ void Filter::autotune(int reps, void* flush, size_t flush_bytes) {
             if (!tile_ok(l, k)) continue;
             c.push_back({time_it([&](cudaStream_t st) { launch_tile(l, k, st); }), kTile, k});
         }
+        if (slab_ok(l)) c.push_back({time_it([&](cudaStream_t st) { launch_slab(l, 0, st); }), kSlab, 0});
         std::stable_sort(c.begin(), c.end(), [](const Choice& a, const Choice& b) { return a.ms < b.ms; });
         v.tuned_path = c[0].path;
         v.tuned_band = c[0].band;
@@ -814,7 +855,7 @@ void Filter::autotune(int reps, void* flush, size_t flush_bytes) {
             };
             for (const Choice& c : timed[l])
                 if (cand[l].size() < 3) cand[l].push_back(c);
-            for (int path : {(int)kStream, (int)kTile}) {
+            for (int path : {(int)kStream, (int)kTile, (int)kSlab}) {
                 int n = 0;
                 for (const Choice& c : timed[l])
                     if (c.path == path && n < 2) {
@@ -970,6 +1011,8 @@ std::string Filter::tuning() const {
             int tw = 0, th = 0;
             tile_shape(v.delta, v.iters, v.smooth, v.W, v.H, param, &tw, &th);
             what = "tile " + std::to_string(tw) + "x" + std::to_string(th);
+        } else if (path == kSlab) {
+            what = "slab " + (param ? std::to_string(param) : std::string("auto"));
         } else {
             what = "per-stage";
         }

@@ -56,7 +56,7 @@ struct Buf {
 enum class Kind { Single = 0, Delta = 1, Pyramidal = 2 };
 
 // how one level step runs
-enum Path { kPerStage = 0, kStream = 1, kTile = 2 };
+enum Path { kPerStage = 0, kStream = 1, kTile = 2, kSlab = 3 };
 
 struct Level {
     bool delta = false;
@@ -78,7 +78,7 @@ struct Level {
     int border = 3;
     bool first = true;
     int tuned_path = -1;         // autotuned: -1 not tuned, else a Path
-    int tuned_band = 0;          // streaming kernel: band rows; tile kernel: tile shape (0 automatic)
+    int tuned_band = 0;          // streaming, slab kernel: band, slab rows; tile kernel: tile shape (0 automatic)
     Buf coarse_rows;             // int per row: coarse row its update reads (delta levels)
     void build_coarse_rows();
     // scratch of the unfused path (allocated on first use)
@@ -146,13 +146,14 @@ public:
     void level_state(int level, int which, void* dst, size_t dst_pitch);
 
     // 0: per-stage kernels only, 1: streaming fused kernel wherever instantiated,
-    // 2: automatic (the autotuned choice, else the streaming kernel for levels of at least
-    // kFusedMinPixels pixels and the tile kernel below), 3: tile-fused kernel wherever it fits
+    // 2: automatic (the autotuned choice, else path_of's rule), 3: tile-fused kernel wherever it
+    // fits
     void set_fused(int mode) {
         fused_mode_ = mode;
         drop_graphs();
     }
-    static constexpr long kFusedMinPixels = 200000;
+    // path_of's rule for untuned levels: streaming kernel from, slab kernel of delta levels from
+    static constexpr long kStreamMinPixels = 1500000, kSlabMinPixels = 76800;
     // time every candidate kernel configuration of each level on the current inputs and
     // keep the fastest (re-running a level step rewrites bit-identical outputs)
     void autotune(int reps, void* flush = nullptr, size_t flush_bytes = 0);
@@ -208,9 +209,12 @@ private:
     void step_level(int l, cudaStream_t s);
     bool fused_ok(int l) const;
     bool tile_ok(int l, int cfg) const;
+    bool slab_ok(int l) const;
     int path_of(int l, int* param) const;
     void launch_fused(int l, int band, cudaStream_t s);
     void launch_tile(int l, int cfg, cudaStream_t s);
+    void launch_slab(int l, int rows, cudaStream_t s);
+    void chain_pdl(int l, LevelArgs& a) const;
     void step_level_unfused(int l, cudaStream_t s);
     void model_unfused(int l, cudaStream_t s);
     void propagate_unfused(int l, cudaStream_t s);

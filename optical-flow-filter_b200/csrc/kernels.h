@@ -63,6 +63,14 @@ struct LevelArgs {
     // finer image (the pyramid step) instead of reading it, and store the tile's pixels of
     // it to img (so every other reader still finds the level image); null otherwise
     const void* pyr_src; size_t pyr_src_pitch; int pyr_src_H, pyr_src_W;
+    // slab kernel, set by its launcher: the state rows (the image rows) allow 16-byte accesses of
+    // four columns
+    int vec, img_vec;
+    // slab kernel, optional (device): the update's gamma, the 5 smoothing weights of the level
+    // (default the 0.2 box), a second copy of the smoothed flow (pitch fs_out_pitch)
+    const float* gamma_dev;
+    const float* weights;
+    float* y_out;
 };
 
 // true if a fused kernel exists for this (delta, item, iterations, smoothing)
@@ -87,6 +95,10 @@ int fused_resident_warps();
 int stream_kind(bool delta, int N, int S);
 int stream_block_smem(bool delta, int S);
 cudaError_t launch_stream_mega(const StreamJob* jobs, int n, int blocks, int smem, cudaStream_t s);
+
+// ---- slab level kernel (slab.cu); LevelArgs::band = output rows of a slab (0 automatic)
+bool slab_available(bool delta, int N, int S);
+cudaError_t launch_slab_level(bool delta, int N, int S, const LevelArgs& a, cudaStream_t s);
 
 // ---- tile-fused per-level kernels (tile_level.cu); cfg 0 = automatic tile shape
 int tile_config_count();
