@@ -509,7 +509,7 @@ ff_status ff_stage_image_model(const void* img, size_t img_pitch, int item_size,
         need(grad, "gradient");
         check_stage_dims(height, width);
         if (item_size != 1 && item_size != 4) throw Error(FF_ERR_INVALID_ARGUMENT, "item size should be 1 or 4");
-        ffb::check_cuda(ffb::launch_image_model(img, img_pitch, item_size, height, width, a0, a0_pitch, grad,
+        ffb::check_cuda(ffb::launch_image_model_stage(img, img_pitch, item_size, height, width, a0, a0_pitch, grad,
                                                 grad_pitch, (cudaStream_t)stream),
                         "image model");
     });
@@ -531,7 +531,7 @@ ff_status ff_stage_propagate(const float* flow, size_t flow_pitch, int height, i
         check_stage_dims(height, width);
         if (iterations <= 0) throw Error(FF_ERR_INVALID_ARGUMENT, "iterations should be greater than zero");
         if (border < 0) throw Error(FF_ERR_INVALID_ARGUMENT, "border should be greater or equal zero");
-        ffb::check_cuda(ffb::launch_propagate(flow, flow_pitch, height, width, iterations, border, out, out_pitch,
+        ffb::check_cuda(ffb::launch_propagate_stage(flow, flow_pitch, height, width, iterations, border, out, out_pitch,
                                               (float*)ws, ws_pitch(width, 8), (cudaStream_t)stream),
                         "propagate");
     });
@@ -563,7 +563,7 @@ ff_status ff_stage_propagate_payload(const float* flow, size_t flow_pitch, const
         float* tf = (float*)base;
         float* tv = (float*)(base + p8 * height);
         float* ts = (float*)(base + 2 * p8 * height);
-        ffb::check_cuda(ffb::launch_propagate_payload(flow, flow_pitch, scalar, scalar_pitch, vector, vector_pitch,
+        ffb::check_cuda(ffb::launch_propagate_payload_stage(flow, flow_pitch, scalar, scalar_pitch, vector, vector_pitch,
                                                       height, width, iterations, border, out_flow, out_flow_pitch,
                                                       out_scalar, out_scalar_pitch, out_vector, out_vector_pitch, tf,
                                                       p8, ts, p4, tv, p8, (cudaStream_t)stream),
@@ -630,7 +630,7 @@ ff_status ff_stage_smooth(const float* flow, size_t flow_pitch, int height, int 
         need(ws, "workspace");
         check_stage_dims(height, width);
         if (iterations <= 0) throw Error(FF_ERR_INVALID_ARGUMENT, "iterations should be greater than zero");
-        ffb::check_cuda(ffb::launch_smooth(flow, flow_pitch, height, width, iterations, out, out_pitch, (float*)ws,
+        ffb::check_cuda(ffb::launch_smooth_stage(flow, flow_pitch, height, width, iterations, out, out_pitch, (float*)ws,
                                            ws_pitch(width, 8), (cudaStream_t)stream),
                         "smooth");
     });

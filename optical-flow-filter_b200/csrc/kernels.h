@@ -45,7 +45,7 @@ struct LevelArgs {
     const float* d_in;   size_t d_in_pitch;    // delta flow (float2), delta levels
     float* fs_out;       size_t fs_out_pitch;
     float* io_out;       size_t io_out_pitch;
-    float* d_out;        size_t d_out_pitch;   // delta levels
+    float* d_out;        size_t d_out_pitch;   // delta levels (slab kernel, top levels: d_in copied, if set)
     float* fu_out;       size_t fu_out_pitch;  // unsmoothed flow (float2), top levels; may be null
     // coarse flow (delta levels)
     const float* coarse; size_t coarse_pitch; int Hc, Wc;
@@ -99,6 +99,30 @@ cudaError_t launch_stream_mega(const StreamJob* jobs, int n, int blocks, int sme
 // ---- slab level kernel (slab.cu); LevelArgs::band = output rows of a slab (0 automatic)
 bool slab_available(bool delta, int N, int S);
 cudaError_t launch_slab_level(bool delta, int N, int S, const LevelArgs& a, cudaStream_t s);
+// the same step of a batch of float images, every field dense (image after image); coarse_rows
+// may be null.  tape (nullable): where to keep the propagated fields (flow, then for delta
+// levels scalar and vector payload, each over the batch) after every X and Y sub-step, the
+// image gradient, and the input of every smoothing pass
+struct SlabTape {
+    float* prop; size_t prop_step;  // sub-step 0; elements to the next
+    float* grad;
+    float* sm; size_t sm_step;      // pass 0's input; elements to the next
+};
+cudaError_t launch_slab_images(bool delta, int N, int S, int images, const LevelArgs& a, const SlabTape* tape,
+                               cudaStream_t s);
+
+// the stages of the stage API: one slab launch for all iterations where it applies (slab.cu),
+// else the per-pass kernels above with their workspaces
+cudaError_t launch_propagate_stage(const float* flow, size_t fp, int H, int W, int N, int border, float* out, size_t op,
+                                   float* tmp, size_t tp, cudaStream_t s);
+cudaError_t launch_propagate_payload_stage(const float* flow, size_t fp, const float* sc, size_t sp, const float* ve,
+                                           size_t vp, int H, int W, int N, int border, float* of, size_t ofp, float* os,
+                                           size_t osp, float* ov, size_t ovp, float* tf, size_t tfp, float* ts, size_t tsp,
+                                           float* tv, size_t tvp, cudaStream_t s);
+cudaError_t launch_smooth_stage(const float* flow, size_t fp, int H, int W, int S, float* out, size_t op, float* tmp,
+                                size_t tp, cudaStream_t s);
+cudaError_t launch_image_model_stage(const void* img, size_t pitch, int item, int H, int W, float* a0, size_t a0p,
+                                     float* grad, size_t gp, cudaStream_t s);
 
 // ---- tile-fused per-level kernels (tile_level.cu); cfg 0 = automatic tile shape
 int tile_config_count();

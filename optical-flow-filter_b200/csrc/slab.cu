@@ -11,6 +11,146 @@ __global__ void __launch_bounds__(32 * kWarps, 1) slab_k(LevelArgs a, Geom g) {
     level_slab<DELTA, P>(a, g, blockIdx.x);
 }
 
+// the same over a batch of float images (every field dense, image after image); TAPE: with the
+// intermediates kept
+template <bool DELTA, bool TAPE>
+__global__ void __launch_bounds__(32 * kWarps, 1) slab_images_k(LevelArgs a, Geom g, int slabs, int images, Tape tape) {
+    const size_t b = blockIdx.x / slabs, n = (size_t)a.H * a.W;
+    auto at = [&](auto*& p, size_t elements) {
+        if (p) p += b * elements;
+    };
+    at(a.fs_in, 2 * n);
+    at(a.io_in, n);
+    at(a.d_in, 2 * n);
+    at(a.fs_out, 2 * n);
+    at(a.io_out, n);
+    at(a.d_out, 2 * n);
+    at(a.fu_out, 2 * n);
+    at(a.y_out, 2 * n);
+    at(a.coarse, 2 * (size_t)a.Hc * a.Wc);
+    a.img = reinterpret_cast<const float*>(a.img) + b * n;
+    at(tape.f, 2 * n);
+    at(tape.s, n);
+    at(tape.v, 2 * n);
+    at(tape.grad, 2 * n);
+    at(tape.sm, 2 * n);
+    level_slab<DELTA, float, TAPE>(a, g, blockIdx.x % slabs, tape);
+}
+
+// The propagation stage alone (FlowPropagator, FlowPropagatorPayload): all N sub-step pairs of a
+// slab in one launch, where the per-pass kernels make 2N round trips through HBM or L2
+template <bool DELTA>
+__global__ void __launch_bounds__(32 * kWarps, 1) propagate_slab_k(LevelArgs a, Geom g) {
+    grid_dep_wait();
+    Ctx c;
+    int sy1;
+    make_ctx<DELTA>(a, g, blockIdx.x, c, sy1);
+    load_state<DELTA>(a, c, sy1);
+    propagate<DELTA, false, true>(c, g.N, g.N, Tape{});
+    grid_dep_launch();
+    if (c.nout <= 0) return;
+    for (int y = c.ys + c.warp; y < c.ye; y += kWarps) {
+        typename Prop<DELTA>::Row r;
+        Prop<DELTA>::load(c.l16 + (unsigned)((y - c.sy0) * Prop<DELTA>::ROWB), r);
+        store_f2(c.vec, c.nout, rowp(reinterpret_cast<float2*>(a.fs_out) + c.c0, (unsigned)a.fs_out_pitch, y), r.q[0], r.q[1]);
+        if constexpr (DELTA) {
+            store_f1(c.vec, c.nout, rowp(a.io_out + c.c0, (unsigned)a.io_out_pitch, y), r.q[2]);
+            store_f2(c.vec, c.nout, rowp(reinterpret_cast<float2*>(a.d_out) + c.c0, (unsigned)a.d_out_pitch, y), r.q[3], r.q[4]);
+        }
+    }
+}
+
+// The smoothing stage alone (FlowSmoother)
+__global__ void __launch_bounds__(32 * kWarps, 1) smooth_slab_k(LevelArgs a, Geom g) {
+    grid_dep_wait();
+    Ctx c;
+    int sy1;
+    make_ctx<false>(a, g, blockIdx.x, c, sy1);
+    load_state<false>(a, c, sy1);
+    grid_dep_launch();
+    smooth<false, false>(c, a, g.S, Tape{});
+}
+
+// The image model stage alone (ImageModel): a warp takes a 128-column window of `rows` rows, the
+// vertical windows in registers; only 4-column halos and 4 rows per run are computed twice.
+template <typename P>
+__global__ void __launch_bounds__(32 * kWarps) image_model_rows_k(const P* __restrict__ img, size_t pitch, int H, int W,
+                                                                 float* __restrict__ a0, size_t a0_pitch,
+                                                                 float2* __restrict__ grad, size_t grad_pitch, int nwx,
+                                                                 int rows) {
+    grid_dep_wait();
+    grid_dep_launch();
+    constexpr int HX = 4, STEP = kCols - 2 * HX;
+    const int w = blockIdx.x * kWarps + (threadIdx.x >> 5);
+    Ctx c;
+    c.W = W;
+    c.H = H;
+    c.lane = threadIdx.x & 31;
+    const int wx = w % nwx, x0 = wx * STEP;
+    c.c0 = x0 + 4 * c.lane;
+    c.ys = w / nwx * rows;
+    c.ye = min(c.ys + rows, H);
+    if (c.ys >= H) return;  // whole warps leave together
+    c.e_l = c.c0 == 0;
+    const bool edge = wx == 0 || wx == nwx - 1;
+    const int xo = wx == 0 ? 0 : x0 + HX, xe = wx == nwx - 1 ? W : x0 + kCols - HX;
+    const int nout = c.c0 >= xo && c.c0 < xe ? min(4, W - c.c0) : 0;
+    const bool vec = nout == 4 && (((uintptr_t)a0 | a0_pitch) % 16) == 0 && (((uintptr_t)grad | grad_pitch) % 32) == 0;
+    // four pixels at once where they are inside and aligned, else one by one at clamped columns
+    const bool word = c.c0 + 3 < W && (((uintptr_t)img | pitch) % (4 * sizeof(P))) == 0;
+    int o[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o[j] = min(c.c0 + j, W - 1);
+    auto load = [&](int y) {
+        const P* r = rowp(img, (unsigned)pitch, min(max(y, 0), H - 1));
+        float v[4];
+        if constexpr (sizeof(P) == 1) {
+            uint32_t q;
+            if (word) q = __ldg(reinterpret_cast<const uint32_t*>(r + c.c0));
+            else q = __ldg(r + o[0]) | __ldg(r + o[1]) << 8 | __ldg(r + o[2]) << 16 | (uint32_t)__ldg(r + o[3]) << 24;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = u8_to_unit((q >> (8 * j)) & 0xffu);
+        } else if (word) {
+            const float4 q = __ldg(reinterpret_cast<const float4*>(r + c.c0));
+            v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = __ldg(r + o[j]);
+        }
+        return Q{make_float2(v[0], v[1]), make_float2(v[2], v[3])};
+    };
+    auto around = [&](const Q& v) {
+        Ext e = extend(v);
+        if (edge) clamp_ext(c, e);  // warp-uniform
+        return e;
+    };
+    Q im[4], bx[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) im[k] = load(c.ys - 2 + k);
+    Q nxt = load(c.ys + 2);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) bx[k] = smooth_x(around(im[k]));
+#pragma unroll 2
+    for (int y = c.ys; y < c.ye; ++y) {
+        const Q i4 = nxt;
+        nxt = load(y + 3);
+        const Q b4 = smooth_x(around(i4));
+        const Ext e = around(smooth_y(im[0], im[1], im[2], im[3], i4));
+        const Q ay = diff_y(bx[0], bx[1], bx[2], bx[3], b4);
+        if (nout > 0) {
+            store_f1(vec, nout, rowp(a0 + c.c0, (unsigned)a0_pitch, y), smooth_x(e));
+            store_f2(vec, nout, rowp(grad + c.c0, (unsigned)grad_pitch, y), diff_x(e), ay);
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            im[k] = im[k + 1];
+            bx[k] = bx[k + 1];
+        }
+        im[3] = i4;
+        bx[3] = b4;
+    }
+}
+
 constexpr int kSmem = 227 * 1024;  // shared memory a block may use on B200
 
 int max_rows(bool delta, int N, int S) {
@@ -36,8 +176,8 @@ Geom geom_of(int N, int S, int W, int H, int rows) {
     Geom g;
     g.N = N;
     g.S = S;
-    const int ox = slab_cols(N, S);
-    g.nwx = (W + ox - 1) / ox;
+    const int step = slab_cols(N, S);
+    g.nwx = 1 + (std::max(W - kCols, 0) + step - 1) / step;
     g.ne = std::min(g.nwx, 2);
     g.rows = std::max(1, std::min(rows, H));
     g.rows_e = std::max(1, std::min((3 * g.rows + 2) / 4, H));
@@ -60,40 +200,89 @@ Geom auto_geom(bool delta, int N, int S, int W, int H, int images) {
     return geom_of(N, S, W, H, hi);
 }
 
-bool rows16(const void* p, size_t pitch, int W, int bytes) {
-    return ((uintptr_t)p | pitch) % 16 == 0 && pitch >= (size_t)((W + 3) & ~3) * bytes;
+// rows of W pixels that may be accessed four pixels (4 * bytes) at a time, up to the next
+// multiple of four columns
+bool rows4(const void* p, size_t pitch, int W, int bytes) {
+    return ((uintptr_t)p | pitch) % (4 * bytes) == 0 && pitch >= (size_t)((W + 3) & ~3) * bytes;
 }
 
-template <bool DELTA, typename P>
-cudaError_t launch(LevelArgs a, int N, int S, cudaStream_t s) {
+// checks and access widths of a launch
+cudaError_t set_access(bool delta, LevelArgs& a) {
     // row offsets are computed as 32 x 32-bit products (rowp)
     for (size_t p : {a.img_pitch, a.fs_in_pitch, a.io_in_pitch, a.d_in_pitch, a.fs_out_pitch, a.io_out_pitch,
                      a.d_out_pitch, a.fu_out_pitch, a.coarse_pitch})
         if (p >> 32) return cudaErrorInvalidPitchValue;
-    a.vec = rows16(a.fs_in, a.fs_in_pitch, a.W, 8) && rows16(a.io_in, a.io_in_pitch, a.W, 4) &&
-            rows16(a.fs_out, a.fs_out_pitch, a.W, 8) && rows16(a.io_out, a.io_out_pitch, a.W, 4) &&
-            (DELTA ? rows16(a.d_in, a.d_in_pitch, a.W, 8) && rows16(a.d_out, a.d_out_pitch, a.W, 8)
-                   : !a.fu_out || rows16(a.fu_out, a.fu_out_pitch, a.W, 8)) &&
-            (!a.y_out || rows16(a.y_out, a.fs_out_pitch, a.W, 8));
+    a.vec = rows4(a.fs_in, a.fs_in_pitch, a.W, 8) && rows4(a.fs_out, a.fs_out_pitch, a.W, 8) &&
+            (!a.io_in || rows4(a.io_in, a.io_in_pitch, a.W, 4)) && (!a.io_out || rows4(a.io_out, a.io_out_pitch, a.W, 4)) &&
+            (delta ? rows4(a.d_in, a.d_in_pitch, a.W, 8) && rows4(a.d_out, a.d_out_pitch, a.W, 8)
+                   : !a.fu_out || rows4(a.fu_out, a.fu_out_pitch, a.W, 8)) &&
+            (!a.y_out || rows4(a.y_out, a.fs_out_pitch, a.W, 8));
     a.img_vec = ((uintptr_t)a.img | a.img_pitch) % 16 == 0;
+    return cudaSuccess;
+}
+
+// once per kernel and device: the shared-memory limit, and the full shared carve-out as for the
+// tile kernels (SMs running small slabs can then also host the other levels' kernels)
+template <auto* K>
+cudaError_t prepare() {
     static std::atomic<unsigned long long> prepared{0};
     int dev = 0;
     cudaGetDevice(&dev);
     const unsigned long long bit = 1ull << (dev & 63);
-    if (!(prepared.load() & bit)) {
-        cudaError_t e = cudaFuncSetAttribute(slab_k<DELTA, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
-        if (e != cudaSuccess) return e;
-        // full shared carve-out, as for the tile kernels: SMs running small slabs can then also
-        // host the other levels' kernels
-        e = cudaFuncSetAttribute(slab_k<DELTA, P>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                 (int)cudaSharedmemCarveoutMaxShared);
-        if (e != cudaSuccess) return e;
-        prepared.fetch_or(bit);
-    }
+    if (prepared.load() & bit) return cudaSuccess;
+    cudaError_t e = cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(K, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
+    if (e == cudaSuccess) prepared.fetch_or(bit);
+    return e;
+}
+
+size_t smem_of(bool delta, const Geom& g) { return (size_t)slab_smem(delta, g.N, g.S, std::max(g.rows, g.rows_e)); }
+
+template <bool DELTA, typename P>
+cudaError_t launch(LevelArgs a, int N, int S, cudaStream_t s) {
+    cudaError_t e = set_access(DELTA, a);
+    if (e == cudaSuccess) e = prepare<slab_k<DELTA, P>>();
+    if (e != cudaSuccess) return e;
     const Geom g = a.band > 0 ? geom_of(N, S, a.W, a.H, std::min(a.band, max_rows(DELTA, N, S)))
                               : auto_geom(DELTA, N, S, a.W, a.H, 1);
-    return launch_k(slab_k<DELTA, P>, dim3(g.slabs(a.H)), dim3(32 * kWarps), (size_t)slab_smem(DELTA, N, S, std::max(g.rows, g.rows_e)),
-                    s, a, g);
+    return launch_k(slab_k<DELTA, P>, dim3(g.slabs(a.H)), dim3(32 * kWarps), smem_of(DELTA, g), s, a, g);
+}
+
+template <bool DELTA>
+cudaError_t launch_propagate_slab(LevelArgs a, int N, cudaStream_t s) {
+    cudaError_t e = set_access(DELTA, a);
+    if (e == cudaSuccess) e = prepare<propagate_slab_k<DELTA>>();
+    if (e != cudaSuccess) return e;
+    const Geom g = auto_geom(DELTA, N, 0, a.W, a.H, 1);
+    return launch_k(propagate_slab_k<DELTA>, dim3(g.slabs(a.H)), dim3(32 * kWarps), smem_of(DELTA, g), s, a, g);
+}
+
+// the rows [p, p + pitch * H) of two fields share memory
+bool overlap(const void* a, size_t ap, const void* b, size_t bp, int H) {
+    const char *x = (const char*)a, *y = (const char*)b;
+    return x < y + bp * H && y < x + ap * H;
+}
+
+// the most sub-step pairs or smoothing iterations of one slab launch
+constexpr int kMaxFused = 8;
+
+template <bool DELTA, bool TAPE>
+cudaError_t launch_images(LevelArgs a, int N, int S, int images, const Tape& tape, cudaStream_t s) {
+    cudaError_t e = set_access(DELTA, a);
+    if (e == cudaSuccess) e = prepare<slab_images_k<DELTA, TAPE>>();
+    if (e != cudaSuccess) return e;
+    // (an image's fields start a multiple of four pixels after the one before where rows may be
+    // accessed by four pixels, so the first image's alignment is every image's)
+    if (TAPE) {
+        auto at = [](const void* p, int bytes) { return (uintptr_t)p % bytes == 0; };
+        a.vec = a.vec && at(tape.f, 32) && at(tape.grad, 32) && at(tape.sm, 32) &&
+                (!DELTA || (at(tape.s, 16) && at(tape.v, 32))) && (tape.step | tape.sm_step) % 8 == 0;
+    }
+    const Geom g = auto_geom(DELTA, N, S, a.W, a.H, images);
+    const int slabs = g.slabs(a.H);
+    return launch_k(slab_images_k<DELTA, TAPE>, dim3((unsigned)slabs * images), dim3(32 * kWarps), smem_of(DELTA, g), s,
+                    a, g, slabs, images, tape);
 }
 
 }  // namespace slab
@@ -104,6 +293,104 @@ cudaError_t launch_slab_level(bool delta, int N, int S, const LevelArgs& a, cuda
     if (!slab_available(delta, N, S)) return cudaErrorInvalidConfiguration;
     if (delta) return a.item == 1 ? slab::launch<true, uint8_t>(a, N, S, s) : slab::launch<true, float>(a, N, S, s);
     return a.item == 1 ? slab::launch<false, uint8_t>(a, N, S, s) : slab::launch<false, float>(a, N, S, s);
+}
+
+cudaError_t launch_slab_images(bool delta, int N, int S, int images, const LevelArgs& a, const SlabTape* tape,
+                               cudaStream_t s) {
+    if (!slab_available(delta, N, S) || a.item != 4) return cudaErrorInvalidConfiguration;
+    slab::Tape t{};
+    if (tape) {
+        const size_t n = (size_t)a.H * a.W * images;
+        t.f = tape->prop;
+        t.s = tape->prop + 2 * n;
+        t.v = tape->prop + 3 * n;
+        t.step = tape->prop_step;
+        t.grad = tape->grad;
+        t.sm = tape->sm;
+        t.sm_step = tape->sm_step;
+        return delta ? slab::launch_images<true, true>(a, N, S, images, t, s)
+                     : slab::launch_images<false, true>(a, N, S, images, t, s);
+    }
+    return delta ? slab::launch_images<true, false>(a, N, S, images, t, s)
+                 : slab::launch_images<false, false>(a, N, S, images, t, s);
+}
+
+// Stage API.  One slab launch instead of 2N (2S) passes, where the outputs share no memory with
+// the inputs (a slab reads its neighbours' rows while they may already be written) and one
+// launch covers the iterations; the per-pass kernels otherwise.  Measured at 1280x720 (device us,
+// against the launches replaced): payload propagation, 4 iterations, 31.1 against 66 (8 launches);
+// smoothing, 2 iterations, 11.7 against 25.8 (4); image model of uint8 8.9 against 23.6, whose
+// one-thread-per-pixel form reads 50 pixels for each
+cudaError_t launch_propagate_stage(const float* flow, size_t fp, int H, int W, int N, int border, float* out, size_t op,
+                                   float* tmp, size_t tp, cudaStream_t s) {
+    if (N > slab::kMaxFused || ((fp | op) >> 32) || slab::overlap(flow, fp, out, op, H))
+        return launch_propagate(flow, fp, H, W, N, border, out, op, tmp, tp, s);
+    LevelArgs a{};
+    a.H = H;
+    a.W = W;
+    a.fs_in = flow, a.fs_in_pitch = fp;
+    a.fs_out = out, a.fs_out_pitch = op;
+    a.border = border;
+    return slab::launch_propagate_slab<false>(a, N, s);
+}
+
+cudaError_t launch_propagate_payload_stage(const float* flow, size_t fp, const float* sc, size_t sp, const float* ve,
+                                           size_t vp, int H, int W, int N, int border, float* of, size_t ofp, float* os,
+                                           size_t osp, float* ov, size_t ovp, float* tf, size_t tfp, float* ts, size_t tsp,
+                                           float* tv, size_t tvp, cudaStream_t s) {
+    const void* in[3] = {flow, sc, ve};
+    const size_t ip[3] = {fp, sp, vp};
+    const void* out[3] = {of, os, ov};
+    const size_t op[3] = {ofp, osp, ovp};
+    bool plain = N > slab::kMaxFused || ((fp | sp | vp | ofp | osp | ovp) >> 32);
+    for (int i = 0; i < 3; ++i)
+        for (int o = 0; o < 3; ++o) plain |= slab::overlap(in[i], ip[i], out[o], op[o], H);
+    if (plain)
+        return launch_propagate_payload(flow, fp, sc, sp, ve, vp, H, W, N, border, of, ofp, os, osp, ov, ovp, tf, tfp, ts,
+                                        tsp, tv, tvp, s);
+    LevelArgs a{};
+    a.H = H;
+    a.W = W;
+    a.fs_in = flow, a.fs_in_pitch = fp;
+    a.io_in = sc, a.io_in_pitch = sp;
+    a.d_in = ve, a.d_in_pitch = vp;
+    a.fs_out = of, a.fs_out_pitch = ofp;
+    a.io_out = os, a.io_out_pitch = osp;
+    a.d_out = ov, a.d_out_pitch = ovp;
+    a.border = border;
+    return slab::launch_propagate_slab<true>(a, N, s);
+}
+
+cudaError_t launch_smooth_stage(const float* flow, size_t fp, int H, int W, int S, float* out, size_t op, float* tmp,
+                                size_t tp, cudaStream_t s) {
+    if (S > slab::kMaxFused || ((fp | op) >> 32) || slab::overlap(flow, fp, out, op, H))
+        return launch_smooth(flow, fp, H, W, S, out, op, tmp, tp, s);
+    LevelArgs a{};
+    a.H = H;
+    a.W = W;
+    a.fs_in = flow, a.fs_in_pitch = fp;
+    a.fs_out = out, a.fs_out_pitch = op;
+    cudaError_t e = slab::set_access(false, a);
+    if (e == cudaSuccess) e = slab::prepare<slab::smooth_slab_k>();
+    if (e != cudaSuccess) return e;
+    const slab::Geom g = slab::auto_geom(false, 0, S, W, H, 1);
+    return launch_k(slab::smooth_slab_k, dim3(g.slabs(H)), dim3(32 * slab::kWarps), slab::smem_of(false, g), s, a, g);
+}
+
+cudaError_t launch_image_model_stage(const void* img, size_t pitch, int item, int H, int W, float* a0, size_t a0p,
+                                     float* grad, size_t gp, cudaStream_t s) {
+    if ((pitch | a0p | gp) >> 32) return launch_image_model(img, pitch, item, H, W, a0, a0p, grad, gp, s);
+    constexpr int step = slab::kCols - 8;
+    const int nwx = 1 + (std::max(W - slab::kCols, 0) + step - 1) / step;
+    // runs of 8 rows (half the vertical windows' work again for their first rows) unless a level
+    // has too few of them to give every SM a block
+    const int rows = (long)nwx * ((H + 7) / 8) >= (long)slab::sm_count() * slab::kWarps ? 8 : 4;
+    const int blocks = (nwx * ((H + rows - 1) / rows) + slab::kWarps - 1) / slab::kWarps;
+    if (item == 1)
+        return launch_k(slab::image_model_rows_k<uint8_t>, dim3(blocks), dim3(32 * slab::kWarps), 0, s, (const uint8_t*)img,
+                        pitch, H, W, a0, a0p, (float2*)grad, gp, nwx, rows);
+    return launch_k(slab::image_model_rows_k<float>, dim3(blocks), dim3(32 * slab::kWarps), 0, s, (const float*)img, pitch, H,
+                    W, a0, a0p, (float2*)grad, gp, nwx, rows);
 }
 
 }  // namespace ffb

@@ -47,6 +47,7 @@ constexpr int kPlane = kCols * 4;   // bytes of one channel of a row
 constexpr int kWarps = 8;           // warps of a slab: the row windows take over 128 registers
 
 __host__ __device__ constexpr int halo_x(int N, int S) { return ((2 * S + (N > 2 ? N : 2)) + 3) & ~3; }
+// columns from a window to the next
 __host__ __device__ constexpr int slab_cols(int N, int S) { return kCols - 2 * halo_x(N, S); }
 // planes of a row: the propagated channels U, V, I, DX, DY (delta levels); U, V and the
 // smoothing passes' second pair (top levels)
@@ -117,11 +118,14 @@ struct Ctx {
     int c0;             // first pixel column of this lane
     int wcol;           // first column of its 4-pixel loads, inside the image
     int ys, ye;         // output rows
+    int nout;           // pixels this lane stores (0 outside the slab's output columns)
+    bool vec;           // all four at once (flow rows 32-byte, scalar rows 16-byte aligned)
     unsigned l16;       // 16 * lane
     int cin;            // bit j: pixel j outside the propagation border columns
     bool e_l, e_r;      // c0 == 0; c0 + 3 == W - 1
     int rag;            // W - 1 - c0 where column W - 1 is pixel 0..2 of this lane, else -1
     bool edge;          // block-uniform: some lane is at an image edge, a border column or outside
+    bool rows_edge;     // block-uniform: edge, or rows of the propagation border
     int sy0;            // first row in shared memory
     unsigned spare;     // the warp's spare row
     // rows of radius r around the output, cut to the image, split over the warps
@@ -130,6 +134,42 @@ struct Ctx {
         y0 = a + n * warp / kWarps;
         y1 = a + n * (warp + 1) / kWarps;
     }
+};
+
+// the slab's output columns of a row: lanes store all four pixels, or (at a ragged right
+// edge, or with unaligned rows) n of them one by one
+__device__ __forceinline__ void store_f2(bool vec, int n, float2* row, const Q& u, const Q& v) {
+    if (vec) {  // one 32-byte store: whole sectors, half the store instructions of 16-byte ones
+        asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(row), "f"(u.a.x), "f"(v.a.x),
+                     "f"(u.a.y), "f"(v.a.y), "f"(u.b.x), "f"(v.b.x), "f"(u.b.y), "f"(v.b.y)
+                     : "memory");
+    } else {
+        if (n > 0) row[0] = make_float2(u.a.x, v.a.x);
+        if (n > 1) row[1] = make_float2(u.a.y, v.a.y);
+        if (n > 2) row[2] = make_float2(u.b.x, v.b.x);
+        if (n > 3) row[3] = make_float2(u.b.y, v.b.y);
+    }
+}
+__device__ __forceinline__ void store_f1(bool vec, int n, float* row, const Q& v) {
+    if (vec) {
+        *reinterpret_cast<float4*>(row) = make_float4(v.a.x, v.a.y, v.b.x, v.b.y);
+    } else {
+        if (n > 0) row[0] = v.a.x;
+        if (n > 1) row[1] = v.a.y;
+        if (n > 2) row[2] = v.b.x;
+        if (n > 3) row[3] = v.b.y;
+    }
+}
+
+// Where a forward that is differentiated later keeps its intermediates, dense images of the
+// level: the propagated channels after every X and Y sub-step, the image gradient, and the
+// input of every smoothing pass.
+struct Tape {
+    float *f, *s, *v;  // sub-step 0's flow, scalar and vector payload (delta levels)
+    size_t step;       // elements from a sub-step to the next
+    float* grad;
+    float* sm;         // smoothing pass 0's input
+    size_t sm_step;
 };
 
 // ---------------------------------------------------------------- propagation
@@ -246,8 +286,9 @@ struct Prop {
     // One sub-step pair over the rows of radius r, in place.  LAST: the pair before the update,
     // which reads only the payload of a delta level, so its flow channels are not computed.
     // E: the slab has lanes at image edges or border columns, or rows of the border.
-    template <bool LAST, bool E>
-    __device__ __forceinline__ static void pass(const Ctx& c, float dt, int r) {
+    // TAPE: X and Y results of the slab's own rows also go to the tape, as sub-steps 2k, 2k + 1.
+    template <bool LAST, bool E, bool TAPE>
+    __device__ __forceinline__ static void pass(const Ctx& c, float dt, int r, const Tape& tape, int k) {
         constexpr int FX = LAST && DELTA ? CV : 0, FY = LAST && DELTA ? 2 : 0;  // first channels of X and Y
         int y0, y1;
         c.run_of(r, y0, y1);
@@ -273,16 +314,28 @@ struct Prop {
             // X of row q + 1 (row `next` of the window), then Y of row q
             unsigned s = base + y0 * ROWB;  // row q + 1
             int q = y0 - 1;
+            auto keep = [&](const Row& v, int y, int sub) {
+                if (TAPE && y >= c.ys && y < c.ye && c.nout > 0) {
+                    const size_t at = (size_t)sub * tape.step, n = (size_t)y * c.W + c.c0;
+                    store_f2(c.vec, c.nout, reinterpret_cast<float2*>(tape.f + at) + n, v.q[0], v.q[1]);
+                    if constexpr (DELTA) {
+                        store_f1(c.vec, c.nout, tape.s + at + n, v.q[2]);
+                        store_f2(c.vec, c.nout, reinterpret_cast<float2*>(tape.v + at) + n, v.q[3], v.q[4]);
+                    }
+                }
+            };
             auto row = [&](const Row& prev, const Row& cur, Row& next) {
                 const bool end = q + 1 == y1;
                 load(end ? spare : s, next);
                 if (inside(end ? yb : q + 1)) xstep<E, FX>(c, dt, next, next);
+                if (!end) keep(next, q + 1, 2 * k);
                 if (q >= y0) {
                     Row y;
                     if (inside(q)) ystep<E, FY>(c, dt, prev, cur, next, y);
                     else y = cur;
 #pragma unroll
                     for (int ch = FY; ch < NC; ++ch) stq(s - ROWB + ch * kPlane, y.q[ch]);
+                    keep(y, q, 2 * k + 1);
                 }
                 s += ROWB;
                 return ++q == y1;
@@ -352,30 +405,6 @@ __device__ __forceinline__ Q smooth_y(const Q& a, const Q& b, const Q& cc, const
 }
 __device__ __forceinline__ Q diff_y(const Q& a, const Q& b, const Q& cc, const Q& d, const Q& e) {
     return Q{diff5_pair(a.a, b.a, cc.a, d.a, e.a), diff5_pair(a.b, b.b, cc.b, d.b, e.b)};
-}
-
-// the window's output columns of a row: lanes store all four pixels, or (at a ragged right
-// edge, or with unaligned rows) n of them one by one
-__device__ __forceinline__ void store_f2(bool vec, int n, float2* row, const Q& u, const Q& v) {
-    if (vec) {
-        reinterpret_cast<float4*>(row)[0] = make_float4(u.a.x, v.a.x, u.a.y, v.a.y);
-        reinterpret_cast<float4*>(row)[1] = make_float4(u.b.x, v.b.x, u.b.y, v.b.y);
-    } else {
-        if (n > 0) row[0] = make_float2(u.a.x, v.a.x);
-        if (n > 1) row[1] = make_float2(u.a.y, v.a.y);
-        if (n > 2) row[2] = make_float2(u.b.x, v.b.x);
-        if (n > 3) row[3] = make_float2(u.b.y, v.b.y);
-    }
-}
-__device__ __forceinline__ void store_f1(bool vec, int n, float* row, const Q& v) {
-    if (vec) {
-        *reinterpret_cast<float4*>(row) = make_float4(v.a.x, v.a.y, v.b.x, v.b.y);
-    } else {
-        if (n > 0) row[0] = v.a.x;
-        if (n > 1) row[1] = v.a.y;
-        if (n > 2) row[2] = v.b.x;
-        if (n > 3) row[3] = v.b.y;
-    }
 }
 
 // ---------------------------------------------------------------- image model and update
@@ -458,7 +487,9 @@ struct Update {
 
     // rows of radius 2S: the model from the image (its vertical windows in registers down the
     // warp's run), the update from the propagated state; the new flow replaces planes U, V
-    __device__ __forceinline__ static void pass(const Ctx& c, const LevelArgs& a, int r2, int nout) {
+    template <bool TAPE>
+    __device__ __forceinline__ static void pass(const Ctx& c, const LevelArgs& a, int r2, const Tape& tape) {
+        const int nout = c.nout;
         int y0, y1;
         c.run_of(r2, y0, y1);
         if (y0 < y1) {
@@ -466,7 +497,7 @@ struct Update {
             const float gamma = a.gamma_dev ? __ldg(a.gamma_dev) : a.gamma;
             const float2 g = make_float2(gamma, gamma);
             const float m = a.maxflow, hm = __fmul_rn(0.5f, m);
-            const bool first = a.first != 0, vec = nout == 4 && a.vec;
+            const bool first = a.first != 0, vec = c.vec;
             float* const io_out = a.io_out + c.c0;
             float2* const f_out = reinterpret_cast<float2*>(DELTA ? a.d_out : a.fu_out) + c.c0;
             const unsigned f_pitch = (unsigned)(DELTA ? a.d_out_pitch : a.fu_out_pitch);
@@ -480,17 +511,26 @@ struct Update {
                 cc[j] = x;
                 cx[j] = DELTA ? 8u * (unsigned)upmap_index(x, c.W, a.Wc) : 0u;
             }
+            auto around = [&](const Q& v) {
+                Ext e = extend(v);
+                if (c.edge) clamp_ext(c, e);  // block-uniform
+                return e;
+            };
             Q im[4], bx[4];
             typename Image<P>::Raw nxt = img.raw(y0 + 2);
             // the coarse flow (delta levels) or old image (top levels) of a row, fetched a row
             // ahead; the coarse row two rows ahead
             float2 u0, u1, u2, u3;
             Q old_top;
-            int crow = DELTA ? __ldg(a.coarse_rows + y0) : 0;
+            // the coarse row of a row, from the level's table where it has one
+            auto coarse_row = [&](int y) {
+                return a.coarse_rows ? __ldg(a.coarse_rows + y) : upmap_index(y, c.H, a.Hc);
+            };
+            int crow = DELTA ? coarse_row(y0) : 0;
             auto fetch = [&](int y) {
                 if constexpr (DELTA) {
                     const char* row = rowp(reinterpret_cast<const char*>(a.coarse), (unsigned)a.coarse_pitch, crow);
-                    crow = __ldg(a.coarse_rows + min(y + 1, c.H - 1));
+                    crow = coarse_row(min(y + 1, c.H - 1));
                     u0 = __ldg(reinterpret_cast<const float2*>(row + cx[0]));
                     u1 = __ldg(reinterpret_cast<const float2*>(row + cx[1]));
                     u2 = __ldg(reinterpret_cast<const float2*>(row + cx[2]));
@@ -510,7 +550,7 @@ struct Update {
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 im[k] = img.unit(img.raw(y0 - 2 + k));
-                bx[k] = smooth_x(extend(im[k]));
+                bx[k] = smooth_x(around(im[k]));
             }
 #pragma unroll 1
             for (int y = y0; y < y1; ++y) {
@@ -521,11 +561,10 @@ struct Update {
                 Q old = DELTA ? ldq(s + 2 * kPlane) : old_top;
                 fetch(y + 1);
                 const Q fx = ldq(s + (DELTA ? 3 : 0) * kPlane), fy = ldq(s + (DELTA ? 4 : 1) * kPlane);
-                // image model (imagemodel_k.cu:31-133); raw columns are loaded clamped, so
-                // nothing is substituted
+                // image model (imagemodel_k.cu:31-133)
                 const Q i4 = img.unit(now);
-                const Q b4 = smooth_x(extend(i4));
-                const Ext e = extend(smooth_y(im[0], im[1], im[2], im[3], i4));
+                const Q b4 = smooth_x(around(i4));
+                const Ext e = around(smooth_y(im[0], im[1], im[2], im[3], i4));
                 const Q ay = diff_y(bx[0], bx[1], bx[2], bx[3], b4);
                 const Q a0 = smooth_x(e), ax = diff_x(e);
 #pragma unroll
@@ -554,6 +593,16 @@ struct Update {
                 if (y >= c.ys && y < c.ye && nout > 0) {
                     store_f1(vec, nout, rowp(io_out, (unsigned)a.io_out_pitch, y), a0);
                     if (f_store) store_f2(vec, nout, rowp(f_out, f_pitch, y), ox, oy);
+                    if (TAPE) {
+                        const size_t n = (size_t)y * c.W + c.c0;
+                        store_f2(vec, nout, reinterpret_cast<float2*>(tape.grad) + n, ax, ay);
+                        store_f2(vec, nout, reinterpret_cast<float2*>(tape.sm) + n, fu, fv);
+                    }
+                    if (!DELTA && a.d_out) {  // a state field that top levels pass on unchanged
+                        const float2* d = rowp(reinterpret_cast<const float2*>(a.d_in), (unsigned)a.d_in_pitch, y) + c.c0;
+                        float2* o = rowp(reinterpret_cast<float2*>(a.d_out), (unsigned)a.d_out_pitch, y) + c.c0;
+                        for (int j = 0; j < nout; ++j) o[j] = __ldg(d + j);
+                    }
                 }
             }
         }
@@ -582,8 +631,9 @@ struct Smooth {
     }
 
     // X: planes U, V -> the next two, rows of radius r + 2
-    template <bool E>
-    __device__ __forceinline__ static void pass_x(const Ctx& c, const W5& w, int r) {
+    // (pass j: the index of what it writes in the tape)
+    template <bool E, bool TAPE>
+    __device__ __forceinline__ static void pass_x(const Ctx& c, const W5& w, int r, const Tape& tape, int j) {
         int y0, y1;
         c.run_of(r + 2, y0, y1);
         unsigned s = (unsigned)((y0 - c.sy0) * ROWB) + c.l16;
@@ -592,15 +642,19 @@ struct Smooth {
             const Q u = box_x<E>(c, w, ldq(s)), v = box_x<E>(c, w, ldq(s + kPlane));
             stq(s + 2 * kPlane, u);
             stq(s + 3 * kPlane, v);
+            if (TAPE && y >= c.ys && y < c.ye && c.nout > 0)
+                store_f2(c.vec, c.nout, reinterpret_cast<float2*>(tape.sm + j * tape.sm_step) + (size_t)y * c.W + c.c0, u, v);
         }
         __syncthreads();
     }
     // Y: back to planes U, V, or (LAST) to the smoothed flow, rows of radius r
-    template <bool LAST>
-    __device__ __forceinline__ static void pass_y(const Ctx& c, const LevelArgs& a, const W5& w, int r, int nout) {
+    template <bool LAST, bool TAPE>
+    __device__ __forceinline__ static void pass_y(const Ctx& c, const LevelArgs& a, const W5& w, int r, const Tape& tape,
+                                                  int j) {
         int y0, y1;
         c.run_of(r, y0, y1);
-        const bool vec = nout == 4 && a.vec;
+        const bool vec = c.vec;
+        const int nout = c.nout;
         float2* const fs_out = reinterpret_cast<float2*>(a.fs_out) + c.c0;
         float2* const y_out = a.y_out ? reinterpret_cast<float2*>(a.y_out) + c.c0 : nullptr;
         const unsigned base = 2 * kPlane + c.l16 - (unsigned)(c.sy0 * ROWB);
@@ -628,6 +682,9 @@ struct Smooth {
                     const unsigned o = base - 2 * kPlane + (unsigned)(y * ROWB);
                     stq(o, ou);
                     stq(o + kPlane, ov);
+                    if (TAPE && y >= c.ys && y < c.ye && nout > 0)
+                        store_f2(vec, nout, reinterpret_cast<float2*>(tape.sm + j * tape.sm_step) + (size_t)y * c.W + c.c0,
+                                 ou, ov);
                 }
             };
             // four rows a turn, so the window rotates without moves
@@ -648,16 +705,12 @@ struct Smooth {
 };
 
 // ---------------------------------------------------------------- one slab
-// slab i of the level step (a, g), by the whole block
-template <bool DELTA, typename P>
-__device__ __forceinline__ void level_slab(const LevelArgs& a, const Geom& g, int i) {
-    // ordering with the preceding kernel: see LevelArgs::pdl_late_wait (everything before the
-    // update reads only the previous frame's state and an image that was complete before)
-    if (!a.pdl_late_wait) grid_dep_wait();
-    if (a.pdl_early_trigger) grid_dep_launch();
+// geometry of slab i: lanes, rows, and which edge handling it needs; sy1 = end of its rows in
+// shared memory
+template <bool DELTA>
+__device__ __forceinline__ void make_ctx(const LevelArgs& a, const Geom& g, int i, Ctx& c, int& sy1) {
     constexpr int ROWB = planes(DELTA) * kPlane;
     const int N = g.N, S = g.S;
-    Ctx c;
     c.W = a.W;
     c.H = a.H;
     c.border = a.border;
@@ -666,8 +719,9 @@ __device__ __forceinline__ void level_slab(const LevelArgs& a, const Geom& g, in
     c.l16 = 16 * c.lane;
     int wx, ys, rows;
     g.at(i, wx, ys, rows);
-    const int HX = halo_x(N, S), OX = kCols - 2 * HX;
-    const int xo = wx * OX, x0 = xo - HX;
+    // window wx starts at column x0; its outer HX columns belong to its neighbours, if it has any
+    const int HX = halo_x(N, S), x0 = wx * slab_cols(N, S);
+    const int xo = wx == 0 ? 0 : x0 + HX, xe = wx == g.nwx - 1 ? a.W : x0 + kCols - HX;
     c.c0 = x0 + 4 * c.lane;
     c.wcol = min(max(c.c0, 0), (c.W - 1) & ~3);
     c.ys = ys;
@@ -680,15 +734,20 @@ __device__ __forceinline__ void level_slab(const LevelArgs& a, const Geom& g, in
 #pragma unroll
     for (int j = 0; j < 4; ++j) c.cin |= (c.c0 + j >= a.border && c.c0 + j < a.W - a.border) << j;
     c.edge = x0 <= 0 || x0 + kCols >= a.W || x0 < a.border || x0 + kCols > a.W - a.border;
-    // pixels this lane stores (0 outside the slab's output columns)
-    const int nout = c.c0 >= xo && c.c0 < xo + OX ? max(0, min(4, a.W - c.c0)) : 0;
+    c.nout = c.c0 >= xo && c.c0 < xe ? min(4, a.W - c.c0) : 0;
+    c.vec = c.nout == 4 && a.vec;
     const int R = N + 2 * S;
     c.sy0 = max(0, ys - R);
-    const int sy1 = min(a.H, c.ye + R);
+    sy1 = min(a.H, c.ye + R);
     c.spare = (unsigned)((sy1 - c.sy0 + c.warp) * ROWB);
-    const bool rows_edge = c.edge || c.sy0 < a.border || sy1 > a.H - a.border;
+    c.rows_edge = c.edge || c.sy0 < a.border || sy1 > a.H - a.border;
 
-    // ---- previous frame's state into the planes, all rows in flight at once
+}
+
+// the previous frame's state of the slab's rows into the planes, all rows in flight at once
+template <bool DELTA>
+__device__ __forceinline__ void load_state(const LevelArgs& a, const Ctx& c, int sy1) {
+    constexpr int ROWB = planes(DELTA) * kPlane;
     {
         const char* fs = reinterpret_cast<const char*>(a.fs_in) + 8 * (size_t)c.wcol;
         const char* d = reinterpret_cast<const char*>(a.d_in) + 8 * (size_t)c.wcol;
@@ -743,35 +802,64 @@ __device__ __forceinline__ void level_slab(const LevelArgs& a, const Geom& g, in
         }
     }
     __syncthreads();
+}
 
-    // ---- propagation, dt = 1/N (FlowPropagator::setIterations, propagation.cu:146-147)
+// N sub-step pairs, dt = 1/N (FlowPropagator::setIterations, propagation.cu:146-147), from rows of
+// radius R.  FULL: every channel of the last pair too (the update reads only the payload of a
+// delta level).
+template <bool DELTA, bool TAPE, bool FULL = TAPE>
+__device__ __forceinline__ void propagate(const Ctx& c, int N, int R, const Tape& tape) {
     const float dt = 1.0f / (float)N;
 #pragma unroll 1
-    for (int k = 1; k < N; ++k) {
-        if (rows_edge) Prop<DELTA>::template pass<false, true>(c, dt, R - k);
-        else Prop<DELTA>::template pass<false, false>(c, dt, R - k);
+    for (int k = 1; k < N + (FULL ? 1 : 0); ++k) {
+        if (c.rows_edge) Prop<DELTA>::template pass<false, true, TAPE>(c, dt, R - k, tape, k - 1);
+        else Prop<DELTA>::template pass<false, false, TAPE>(c, dt, R - k, tape, k - 1);
     }
-    if (rows_edge) Prop<DELTA>::template pass<true, true>(c, dt, 2 * S);
-    else Prop<DELTA>::template pass<true, false>(c, dt, 2 * S);
+    if (!FULL) {
+        if (c.rows_edge) Prop<DELTA>::template pass<true, true, false>(c, dt, R - N, tape, N - 1);
+        else Prop<DELTA>::template pass<true, false, false>(c, dt, R - N, tape, N - 1);
+    }
+}
 
-    // ---- image model and update
-    if (a.pdl_late_wait) grid_dep_wait();
-    Update<DELTA, P>::pass(c, a, 2 * S, nout);
-    // the next kernel in the stream may start scheduling its blocks from here on
-    if (!a.pdl_early_trigger) grid_dep_launch();
-
-    // ---- smoothing
+// S smoothing iterations of planes U, V; the last stores the smoothed flow
+template <bool DELTA, bool TAPE>
+__device__ __forceinline__ void smooth(const Ctx& c, const LevelArgs& a, int S, const Tape& tape) {
     typename Smooth<DELTA>::W5 w;
 #pragma unroll
     for (int j = 0; j < 5; ++j) w.k[j] = a.weights ? __ldg(a.weights + j) : kBox;
 #pragma unroll 1
     for (int s = 1; s <= S; ++s) {
         const int r = 2 * (S - s);
-        if (c.edge) Smooth<DELTA>::template pass_x<true>(c, w, r);
-        else Smooth<DELTA>::template pass_x<false>(c, w, r);
-        if (s < S) Smooth<DELTA>::template pass_y<false>(c, a, w, r, nout);
-        else Smooth<DELTA>::template pass_y<true>(c, a, w, r, nout);
+        if (c.edge) Smooth<DELTA>::template pass_x<true, TAPE>(c, w, r, tape, 2 * s - 1);
+        else Smooth<DELTA>::template pass_x<false, TAPE>(c, w, r, tape, 2 * s - 1);
+        if (s < S) Smooth<DELTA>::template pass_y<false, TAPE>(c, a, w, r, tape, 2 * s);
+        else Smooth<DELTA>::template pass_y<true, TAPE>(c, a, w, r, tape, 2 * s);
     }
+}
+
+// slab i of the level step (a, g), by the whole block
+template <bool DELTA, typename P, bool TAPE = false>
+__device__ __forceinline__ void level_slab(const LevelArgs& a, const Geom& g, int i, const Tape& tape = Tape{}) {
+    // ordering with the preceding kernel: see LevelArgs::pdl_late_wait (everything before the
+    // update reads only the previous frame's state and an image that was complete before)
+    if (!a.pdl_late_wait) grid_dep_wait();
+    if (a.pdl_early_trigger) grid_dep_launch();
+    const int N = g.N, S = g.S;
+    Ctx c;
+    int sy1;
+    make_ctx<DELTA>(a, g, i, c, sy1);
+    const int R = N + 2 * S;
+    load_state<DELTA>(a, c, sy1);
+
+    propagate<DELTA, TAPE>(c, N, R, tape);
+
+    // ---- image model and update
+    if (a.pdl_late_wait) grid_dep_wait();
+    Update<DELTA, P>::template pass<TAPE>(c, a, 2 * S, tape);
+    // the next kernel in the stream may start scheduling its blocks from here on
+    if (!a.pdl_early_trigger) grid_dep_launch();
+
+    smooth<DELTA, TAPE>(c, a, S, tape);
 }
 
 }  // namespace slab

@@ -15,7 +15,7 @@ def frames_of(H, W, T, seed):
     k = np.ones(3) / 3
     b = np.apply_along_axis(lambda r: np.convolve(r, k, "same"), 1, base.astype(np.float64))
     b = np.apply_along_axis(lambda r: np.convolve(r, k, "same"), 0, b)
-    return [np.clip(b[t:t + H, t // 2:t // 2 + W], 0, 255).astype(np.uint8) for t in range(T)]
+    return [np.ascontiguousarray(np.clip(b[t:t + H, t // 2:t // 2 + W], 0, 255).astype(np.uint8)) for t in range(T)]
 
 
 def states(f, levels):
@@ -111,3 +111,61 @@ def test_slab_delta_filter(cuda, dtype):
         out.append(got)
     for a, b in zip(*out):
         assert same(a, b)
+
+
+def clip_flows(torch, H, W, n, seed, pad=0):
+    """n float32 fields (H, W, 2) of signed flows with zeros, rows padded by ``pad`` pixels."""
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    out = []
+    for _ in range(n):
+        f = torch.randn((H, W + pad, 2), generator=g, device="cuda")
+        f[torch.rand((H, W + pad), generator=g, device="cuda") < 0.1] = 0.0
+        out.append(f[:, :W])
+    return out
+
+
+@pytest.mark.parametrize("H,W,pad", [(1, 1, 0), (3, 2, 1), (40, 127, 0), (29, 128, 0), (33, 129, 3), (75, 241, 0),
+                                     (260, 116, 4)])
+@pytest.mark.parametrize("n,border", [(1, 0), (2, 3), (5, 1), (8, 3), (9, 3)])
+def test_stages_equal_the_oracle(cuda, H, W, pad, n, border):
+    """Propagation, smoothing and image model at slab edges, at the most iterations of one launch
+    and one more, on padded rows."""
+    import oracle as O
+    from flowfilter_b200 import stages
+
+    torch = cuda
+    flow, vec = clip_flows(torch, H, W, 2, 7 * H + n, pad)
+    sca = torch.rand((H, W + pad), generator=torch.Generator(device="cuda").manual_seed(H + n), device="cuda")[:, :W]
+    host = [t.cpu().numpy().copy() for t in (flow, sca, vec)]
+    got = stages.propagate(flow, n, border).cpu().numpy()
+    assert np.array_equal(got, O.propagate(host[0], n, border))
+    got = [t.cpu().numpy() for t in stages.propagate_payload(flow, sca, vec, n, border)]
+    assert all(np.array_equal(x, y) for x, y in zip(got, O.propagate_payload(*host, n, border)))
+    assert np.array_equal(stages.smooth(flow, n).cpu().numpy(), O.smooth(host[0], n))
+    u8 = torch.from_numpy(frames_of(H, W + pad, 1, n)[0]).cuda()[:, :W]
+    for img in (u8, u8.float() / 255):
+        a0, grad = (t.cpu().numpy() for t in stages.image_model(img))
+        wa, wg = O.image_model(img.cpu().numpy().copy())
+        assert np.array_equal(a0, wa) and np.array_equal(grad, wg)
+
+
+@pytest.mark.parametrize("B,H,W,levels", [(1, 37, 53, 1), (3, 33, 128, 2), (1, 31, 132, 2), (2, 70, 240, 3)])
+def test_taped_frame_equals_the_stage_functions(cuda, B, H, W, levels):
+    """Flows and gradients of the frame node, whose float forward keeps its tape from the slab
+    kernel, against one autograd node per stage."""
+    from flowfilter_b200 import diff
+
+    torch = cuda
+    g = torch.Generator(device="cuda").manual_seed(W)
+    frames = torch.rand((B, 3, H, W), generator=g, device="cuda")
+    res = []
+    for per_stage in (True, False):
+        f = diff.DiffPyramidalFlowFilter(H, W, levels, [0.01, 0.02, 0.03][:levels], [2, 1, 3][:levels], maxflow=3.0)
+        f.per_stage = per_stage
+        x = frames.clone().requires_grad_(True)
+        y = f(x)
+        y.square().sum().backward()
+        res.append((y.detach(), f.gamma.grad, f.weights.grad, x.grad))
+    assert torch.equal(res[0][0], res[1][0])
+    for a, b in zip(res[0][1:], res[1][1:]):  # the same sums in another order
+        assert torch.allclose(a, b, rtol=1e-3, atol=1e-5 * float(a.abs().max()))
