@@ -224,6 +224,17 @@ def call(name: str, *args) -> None:
     check(getattr(lib(), name)(*args))
 
 
+def current_stream() -> int:
+    """The handle of torch's current stream on the current device.  torch.cuda.current_stream()
+    builds a Stream object on each call (3.3 us of a small frame's 29); the handle alone takes a
+    tenth of that."""
+    import torch
+
+    if torch.cuda.is_initialized():
+        return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    return torch.cuda.current_stream().cuda_stream
+
+
 _log_callback = None  # the ctypes thunk the library holds, kept alive here
 
 

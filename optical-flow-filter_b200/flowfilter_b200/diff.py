@@ -21,7 +21,7 @@ from __future__ import annotations
 import ctypes
 import math
 
-from ._lib import call, lib
+from ._lib import call, current_stream, lib
 
 
 def _torch():
@@ -35,7 +35,7 @@ def _dt(x) -> int:
 
 
 def _stream():
-    return ctypes.c_void_p(_torch().cuda.current_stream().cuda_stream)
+    return ctypes.c_void_p(current_stream())
 
 
 def _p(t):

@@ -15,7 +15,7 @@ import ctypes
 import numpy as np
 
 from . import _lib
-from ._lib import FFImage, call, lib
+from ._lib import FFImage, call, current_stream, lib
 
 __all__ = ["FlowFilter", "PyramidalFlowFilter", "DeltaFlowFilter", "BatchFlowFilter", "device_view"]
 
@@ -83,6 +83,7 @@ def _host_array(x, dtype, shape) -> np.ndarray:
 
 class _FilterBase:
     _h = None
+    _dims = None  # (height, width, levels), fixed when the filter is made
 
     def __del__(self):
         h, self._h = getattr(self, "_h", None), None
@@ -91,9 +92,11 @@ class _FilterBase:
 
     # ------------------------------------------------------------ helpers
     def _shape(self):
-        h, w, l = ctypes.c_int(), ctypes.c_int(), ctypes.c_int()
-        call("ff_filter_shape", self._h, ctypes.byref(h), ctypes.byref(w), ctypes.byref(l))
-        return h.value, w.value, l.value
+        if self._dims is None:
+            h, w, l = ctypes.c_int(), ctypes.c_int(), ctypes.c_int()
+            call("ff_filter_shape", self._h, ctypes.byref(h), ctypes.byref(w), ctypes.byref(l))
+            self._dims = h.value, w.value, l.value
+        return self._dims
 
     def _item(self) -> int:
         return 1
@@ -105,12 +108,12 @@ class _FilterBase:
         if _is_torch(img) and img.is_cuda:
             torch = _torch()
             want = torch.uint8 if dtype == np.uint8 else torch.float32
-            if img.dtype != want or tuple(img.shape) != (self.height, self.width):
+            if img.dtype != want or img.shape != self._shape()[:2]:
                 raise ValueError(f"expected a {want} tensor of shape {(self.height, self.width)}, "
                                  f"got {img.dtype} {tuple(img.shape)}")
             if img.stride(1) != 1:
                 img = img.contiguous()
-            stream = torch.cuda.current_stream().cuda_stream
+            stream = current_stream()
             call("ff_filter_load_image_device_async", self._h, ctypes.c_void_p(img.data_ptr()),
                  img.stride(0) * img.element_size(), ctypes.c_void_p(stream))
             self._keep_input = img
@@ -132,7 +135,7 @@ class _FilterBase:
     def computeAsync(self, stream=None) -> None:
         """Enqueue one frame on ``stream`` (default: the current torch stream)."""
         if stream is None:
-            stream = _torch().cuda.current_stream().cuda_stream
+            stream = current_stream()
         elif hasattr(stream, "cuda_stream"):
             stream = stream.cuda_stream
         call("ff_filter_compute_async", self._h, ctypes.c_void_p(stream))
@@ -148,7 +151,7 @@ class _FilterBase:
         img_in, _ = _host_image(fin, 1)
         img_out, _ = _host_image(fout, 2)
         if stream is None:
-            stream = _torch().cuda.current_stream().cuda_stream if _torch_cuda() else 0
+            stream = current_stream() if _torch_cuda() else 0
         elif hasattr(stream, "cuda_stream"):
             stream = stream.cuda_stream
         call("ff_filter_process_host_async", self._h, ctypes.byref(img_in), ctypes.byref(img_out),
@@ -201,7 +204,8 @@ class _FilterBase:
     def _device_result(self, which: int, channels: int):
         p, pitch = ctypes.c_void_p(), ctypes.c_size_t()
         call("ff_filter_device_result", self._h, which, ctypes.byref(p), ctypes.byref(pitch))
-        return device_view(p.value, pitch.value, self.height, self.width, channels, owner=self)
+        h, w, _ = self._shape()
+        return device_view(p.value, pitch.value, h, w, channels, owner=self)
 
     def getFlowDevice(self):
         """torch view of getFlow() on the device (valid until the next compute)."""
@@ -750,7 +754,7 @@ class BatchFlowFilter:
                 and frames.numel() >= self._total):
             raise ValueError(f"frames should be a contiguous uint8 CUDA tensor of {self._total} bytes")
         if stream is None:
-            stream = torch.cuda.current_stream().cuda_stream
+            stream = current_stream()
         elif hasattr(stream, "cuda_stream"):
             stream = stream.cuda_stream
         call("ff_batch_step", self._h, ctypes.c_void_p(frames.data_ptr()), ctypes.c_void_p(stream))

@@ -23,7 +23,7 @@ import ctypes
 
 import numpy as np
 
-from ._lib import call, lib
+from ._lib import call, current_stream, lib
 
 __all__ = ["GPUImage", "ImageModel", "ImagePyramid", "FlowPropagator", "FlowPropagatorPayload", "FlowUpdate",
            "DeltaFlowUpdate", "FlowSmoother"]
@@ -36,7 +36,7 @@ def _torch():
 
 
 def _stream():
-    return ctypes.c_void_p(_torch().cuda.current_stream().cuda_stream)
+    return ctypes.c_void_p(current_stream())
 
 
 def _p(t):

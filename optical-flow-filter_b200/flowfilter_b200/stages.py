@@ -11,7 +11,7 @@ from __future__ import annotations
 
 import ctypes
 
-from ._lib import call, lib
+from ._lib import call, current_stream, lib
 
 __all__ = ["pyramid_down", "image_model", "propagate", "propagate_payload", "update", "delta_update", "smooth"]
 
@@ -23,7 +23,7 @@ def _torch():
 
 
 def _stream():
-    return ctypes.c_void_p(_torch().cuda.current_stream().cuda_stream)
+    return ctypes.c_void_p(current_stream())
 
 
 def _ptr(t):
