@@ -284,6 +284,7 @@ struct Batch::Table {
     PyrJob* d_pyr = nullptr;
     TileJob* d_tile = nullptr;
     StreamJob* d_stream = nullptr;
+    SlabJob* d_slab = nullptr;
     cudaGraphExec_t graph = nullptr;
     int launches = 0;  // kernel launches of the graph
 };
@@ -371,6 +372,7 @@ void Batch::release_table(Table& t) {
     if (t.d_pyr) cudaFree(t.d_pyr);
     if (t.d_tile) cudaFree(t.d_tile);
     if (t.d_stream) cudaFree(t.d_stream);
+    if (t.d_slab) cudaFree(t.d_slab);
     t = Table{};
 }
 
@@ -412,6 +414,71 @@ bool Batch::streamed(const Filter& f, int l) const {
     const long min_px = min_px_ >= 0 ? min_px_ : kDefaultTileBelow;
     return v.item == 1 && (late || (long)v.H * v.W >= min_px) && f.streaming_ok(l);
 }
+
+// Levels of phase A (0: tops and levels 0..L-3) or phase B (1: levels L-2).  Below kSlabBelow
+// pixels a phase's streaming warps are too few or their bands too short.  Measured step times (us,
+// slab / streaming and tile): 4 streams of 640x480, 2 levels (1.2 M pixels) 91 / 125; 16 of them
+// (4.9 M) 303 / 344; 8 of 1280x720 with 3 levels (7.4 M) 471 / 497; 16 of them (14.7 M) 888 / 785;
+// the 64-stream mix of 54 M pixels 2349 / 2107.
+bool Batch::slab_phase(int phase) const {
+    if (min_px_ >= 0 || band_ > 0 || !level_band_.empty()) return false;
+    long px = 0;
+    for (auto& f : f_) {
+        const int L = f->levels();
+        for (int l = 0; l < L; ++l) {
+            if ((L >= 2 && l == L - 2) != (phase == 1)) continue;
+            const Level& v = f->level(l);
+            px += (long)v.H * v.W;
+            if (px >= kSlabBelow || !f->slab_usable(l)) return false;
+        }
+    }
+    return true;
+}
+
+namespace {
+// Slabs of a phase's jobs: every slab the same time t, as short as lets all of them run at once
+// (one per SM), or in as few waves as their most rows allow.  A slab's time is taken as its
+// rows plus the halo rows it also works on (N + 2S on average over the stages) times the
+// instructions of a row: 185 (delta) or 80 per sub-step pair, 330 for model and update, 110
+// per smoothing iteration.
+struct SlabPlan {
+    struct Item {
+        Filter* f;
+        int l, cls;
+        double cost;
+    };
+    std::vector<Item> items;
+    static int rows_at(const Item& it, double t) {
+        const Level& v = it.f->level(it.l);
+        const int most = std::min(slab_max_rows(v.delta, v.iters, v.smooth), v.H);
+        return std::max(1, std::min((int)(t / it.cost) - (v.iters + 2 * v.smooth), most));
+    }
+    long slabs_at(double t) const {
+        long n = 0;
+        SlabJob j;
+        for (const Item& it : items) {
+            const Level& v = it.f->level(it.l);
+            n += slab_job(j, v.delta, v.iters, v.smooth, it.f->level_args(it.l), rows_at(it, t), nullptr);
+        }
+        return n;
+    }
+    double time(int sms) const {
+        double hi = 0;
+        for (const Item& it : items) {
+            const Level& v = it.f->level(it.l);
+            hi = std::max(hi, it.cost * (v.H + v.iters + 2 * v.smooth + 1));
+        }
+        const long most = (slabs_at(hi) + sms - 1) / sms * sms;
+        double lo = 0;
+        for (int k = 0; k < 24; ++k) {
+            const double mid = 0.5 * (lo + hi);
+            if (slabs_at(mid) <= most) hi = mid;
+            else lo = mid;
+        }
+        return hi;
+    }
+};
+}  // namespace
 
 void Batch::set_tuning(long min_pixels, int band) {
     min_px_ = min_pixels < 0 ? -1 : min_pixels;
@@ -516,6 +583,40 @@ void Batch::build(Table& t) {
     // phase's streaming launch, the others to its tile launch.
     std::vector<StreamJob> sj[2];
     std::vector<TileJob> tj[2];
+    // slab phases: the levels that would stream in sl[ph][0], the others in sl[ph][1]
+    std::vector<SlabJob> sl[2][2];
+    int slblocks[2][2] = {};
+    size_t slsmem[2][2] = {};
+    for (int ph = 0; ph < 2; ++ph) {
+        if (!slab_phase(ph)) continue;
+        SlabPlan plan;
+        for (auto& f : f_) {
+            const int L = f->levels();
+            for (int l = 0; l < L; ++l) {
+                if ((L >= 2 && l == L - 2) != (ph == 1)) continue;
+                const Level& v = f->level(l);
+                plan.items.push_back({f.get(), l, streamed(*f, l) ? 0 : 1,
+                                      (v.delta ? 185.0 : 80.0) * v.iters + 330.0 + 110.0 * v.smooth});
+            }
+        }
+        if (plan.items.empty()) continue;
+        int dev = 0, sms = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        const double t_slab = plan.time(sms > 0 ? sms : 148);
+        for (const auto& it : plan.items) {
+            const Level& v = it.f->level(it.l);
+            SlabJob j{};
+            size_t smem = 0;
+            const int n = slab_job(j, v.delta, v.iters, v.smooth, it.f->level_args(it.l),
+                                   SlabPlan::rows_at(it, t_slab), &smem);
+            if (n <= 0) throw Error(FF_ERR_UNSUPPORTED, "batch: image rows of 4 GB or more");
+            j.first_block = slblocks[ph][it.cls];
+            slblocks[ph][it.cls] += n;
+            slsmem[ph][it.cls] = std::max(slsmem[ph][it.cls], smem);
+            sl[ph][it.cls].push_back(j);
+        }
+    }
     int sblocks[2] = {0, 0}, ssmem[2] = {0, 0}, tblocks[2] = {0, 0};
     size_t tsmem[2] = {0, 0};
     for (auto& fp : f_) {
@@ -524,6 +625,7 @@ void Batch::build(Table& t) {
         for (int l = 0; l < L; ++l) {
             const Level& v = f->level(l);
             const int ph = L >= 2 && l == L - 2 ? 1 : 0;
+            if (!sl[ph][0].empty() || !sl[ph][1].empty()) continue;
             if (streamed(*f, l)) {
                 StreamJob j{};
                 j.a = f->level_args(l);
@@ -572,6 +674,14 @@ void Batch::build(Table& t) {
     t.d_pyr = to_device(pyr);
     t.d_tile = to_device(tall);
     t.d_stream = to_device(sall);
+    std::vector<SlabJob> slall;
+    size_t slfirst[2][2] = {};
+    for (int ph = 0; ph < 2; ++ph)
+        for (int k = 0; k < 2; ++k) {
+            slfirst[ph][k] = slall.size();
+            slall.insert(slall.end(), sl[ph][k].begin(), sl[ph][k].end());
+        }
+    t.d_slab = to_device(slall);
     t.parity.clear();
     t.gen.clear();
     for (auto& f : f_) {
@@ -596,7 +706,7 @@ void Batch::build(Table& t) {
             ++launches;
         }
     for (int ph = 0; ph < 2; ++ph) {
-        const bool branch = ph == 0 && !tj[0].empty() && !sj[0].empty();
+        const bool branch = (ph == 0 && !tj[0].empty() && !sj[0].empty()) || (!sl[ph][0].empty() && !sl[ph][1].empty());
         if (branch) {
             ok(cudaEventRecord(fork_, cap_));
             ok(cudaStreamWaitEvent(side_, fork_, 0));
@@ -609,6 +719,12 @@ void Batch::build(Table& t) {
         if (!tj[ph].empty()) {
             ok(launch_k(tile_batch_k, dim3(tblocks[ph]), dim3(kTileThreads), tsmem[ph], branch ? side_ : cap_,
                         (const TileJob*)(t.d_tile + (ph ? tj[0].size() : 0)), (int)tj[ph].size()));
+            ++launches;
+        }
+        for (int k = 0; k < 2; ++k) {
+            if (sl[ph][k].empty()) continue;
+            ok(launch_slab_jobs(t.d_slab + slfirst[ph][k], (int)sl[ph][k].size(), slblocks[ph][k], slsmem[ph][k],
+                                branch && k == 1 ? side_ : cap_));
             ++launches;
         }
         if (branch) {

@@ -56,6 +56,10 @@ public:
     // (<= 0: chosen per step)
     void set_tuning(long min_pixels, int band);
     static constexpr long kDefaultTileBelow = 200000;
+    // A phase of less than kSlabBelow pixels runs its levels by the slab kernel, in the launches
+    // that otherwise are its streaming and its tile launch, unless set_tuning or set_level_band
+    // ask for something else
+    static constexpr long kSlabBelow = 8000000;
     // levels of height x width pixels run in bands of `band` rows (<= 0: no override)
     void set_level_band(int height, int width, int band);
 
@@ -66,6 +70,7 @@ private:
     bool matches(const Table& t) const;
     void release_table(Table& t);
     bool streamed(const Filter& f, int l) const;
+    bool slab_phase(int phase) const;
     int band_of(const Level& v, int rule_band) const;
 
     std::vector<std::unique_ptr<Filter>> f_;

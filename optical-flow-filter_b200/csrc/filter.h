@@ -191,6 +191,8 @@ public:
     int parity() const { return cur_; }
     // can level l run the streaming fused kernel (instantiated, aligned rows, coarse flow)?
     bool streaming_ok(int l) const { return fused_ok(l); }
+    // can level l run the slab kernel?
+    bool slab_usable(int l) const { return slab_ok(l); }
     // block until everything queued on the filter so far has finished
     void wait_done() const;
     // changes whenever a parameter that shapes the level steps changes

@@ -111,6 +111,21 @@ struct SlabTape {
 cudaError_t launch_slab_images(bool delta, int N, int S, int images, const LevelArgs& a, const SlabTape* tape,
                                cudaStream_t s);
 
+// one level of a batched slab launch (uint8 images): its arguments, its slabs and the first of
+// its blocks
+struct SlabJob {
+    LevelArgs a;
+    int N, S, nwx, rows, rows_e, nby_e, ne;  // slab::Geom
+    int delta;
+    int first_block;
+};
+// output rows a slab can have at most
+int slab_max_rows(bool delta, int N, int S);
+// fills a job (all but first_block) for slabs of `rows` output rows; returns its blocks and the
+// shared memory of one, 0 if the level's pitches are beyond the kernel's reach
+int slab_job(SlabJob& j, bool delta, int N, int S, const LevelArgs& a, int rows, size_t* smem);
+cudaError_t launch_slab_jobs(const SlabJob* jobs, int n, int blocks, size_t smem, cudaStream_t s);
+
 // the stages of the stage API: one slab launch for all iterations where it applies (slab.cu),
 // else the per-pass kernels above with their workspaces
 cudaError_t launch_propagate_stage(const float* flow, size_t fp, int H, int W, int N, int border, float* out, size_t op,

@@ -11,6 +11,21 @@ __global__ void __launch_bounds__(32 * kWarps, 1) slab_k(LevelArgs a, Geom g) {
     level_slab<DELTA, P>(a, g, blockIdx.x);
 }
 
+// level steps of many streams and levels in one launch; a block finds its job by binary search
+__global__ void __launch_bounds__(32 * kWarps, 1) slab_jobs_k(const SlabJob* __restrict__ jobs, int n) {
+    int lo = 0, hi = n - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (jobs[mid].first_block <= (int)blockIdx.x) lo = mid;
+        else hi = mid - 1;
+    }
+    const SlabJob& j = jobs[lo];
+    const Geom g{j.N, j.S, j.nwx, j.rows, j.rows_e, j.nby_e, j.ne};
+    const int i = (int)blockIdx.x - j.first_block;
+    if (j.delta) level_slab<true, uint8_t>(j.a, g, i);
+    else level_slab<false, uint8_t>(j.a, g, i);
+}
+
 // the same over a batch of float images (every field dense, image after image); TAPE: with the
 // intermediates kept
 template <bool DELTA, bool TAPE>
@@ -286,6 +301,30 @@ cudaError_t launch_images(LevelArgs a, int N, int S, int images, const Tape& tap
 }
 
 }  // namespace slab
+
+int slab_max_rows(bool delta, int N, int S) { return slab::max_rows(delta, N, S); }
+
+int slab_job(SlabJob& j, bool delta, int N, int S, const LevelArgs& a, int rows, size_t* smem) {
+    j.a = a;
+    j.delta = delta ? 1 : 0;
+    if (slab::set_access(delta, j.a) != cudaSuccess) return 0;
+    const slab::Geom g = slab::geom_of(N, S, a.W, a.H, std::min(rows, slab::max_rows(delta, N, S)));
+    j.N = N;
+    j.S = S;
+    j.nwx = g.nwx;
+    j.rows = g.rows;
+    j.rows_e = g.rows_e;
+    j.nby_e = g.nby_e;
+    j.ne = g.ne;
+    if (smem) *smem = slab::smem_of(delta, g);
+    return g.slabs(a.H);
+}
+
+cudaError_t launch_slab_jobs(const SlabJob* jobs, int n, int blocks, size_t smem, cudaStream_t s) {
+    const cudaError_t e = slab::prepare<slab::slab_jobs_k>();
+    if (e != cudaSuccess) return e;
+    return launch_k(slab::slab_jobs_k, dim3(blocks), dim3(32 * slab::kWarps), smem, s, jobs, n);
+}
 
 bool slab_available(bool delta, int N, int S) { return N >= 1 && S >= 1 && slab::max_rows(delta, N, S) >= 1; }
 
