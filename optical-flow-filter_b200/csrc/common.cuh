@@ -105,10 +105,10 @@ __device__ __forceinline__ void pyramid_px(const CView<P>& in, const View<P>& ou
     out.at(x, y) = pyramid_val(in, x, y);
 }
 
-// dominant velocity: |v+| - |v-| > 0 ? v+ : v-   (propagation_k.cu:37-40)
-__device__ __forceinline__ float dominant(float vm, float vp) {
-    return __fsub_rn(fabsf(vp), fabsf(vm)) > 0.0f ? vp : vm;
-}
+// dominant velocity: |v+| - |v-| > 0 ? v+ : v-   (propagation_k.cu:37-40).  The difference is
+// positive exactly where |v+| > |v-| (denormals are kept; inf - inf and NaN give false both
+// ways), so one comparison does.
+__device__ __forceinline__ float dominant(float vm, float vp) { return fabsf(vp) > fabsf(vm) ? vp : vm; }
 
 // One upwind sub-step f0 - t*(dv >= 0 ? f0 - fm : fp - f0), t = dt*dv
 // (propagation_k.cu:50-53, 175-207).  The reference build fuses the multiply into the

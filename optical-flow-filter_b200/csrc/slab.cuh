@@ -194,9 +194,6 @@ struct Prop {
         if (FUSED) return make_float2(__fmaf_rn(nat.x, dx, v.x), __fmaf_rn(nat.y, dy, v.y));
         return make_float2(__fadd_rn(v.x, __fmul_rn(nat.x, dx)), __fadd_rn(v.y, __fmul_rn(nat.y, dy)));
     }
-    // dominant velocity: |v+| - |v-| > 0 exactly where |v+| > |v-| (no flush to zero)
-    __device__ __forceinline__ static float dom(float vm, float vp) { return fabsf(vp) > fabsf(vm) ? vp : vm; }
-
     // the neighbour before pixel 0 and after pixel 3, clamped at the image edges (E)
     template <bool E>
     __device__ __forceinline__ static void around(const Ctx& c, const Q& v, float& L, float& R) {
@@ -220,8 +217,8 @@ struct Prop {
         auto right1 = [&](int ch) { return E && c.rag == 1 ? v.q[ch].a.y : v.q[ch].b.x; };
         auto right2 = [&](int ch) { return E && c.rag == 2 ? v.q[ch].b.x : v.q[ch].b.y; };
         const Q& u = v.q[CU];
-        const float v0 = dom(L[CU], right0(CU)), v1 = dom(u.a.x, right1(CU));
-        const float v2 = dom(u.a.y, right2(CU)), v3 = dom(u.b.x, R[CU]);
+        const float v0 = dominant(L[CU], right0(CU)), v1 = dominant(u.a.x, right1(CU));
+        const float v2 = dominant(u.a.y, right2(CU)), v3 = dominant(u.b.x, R[CU]);
         const bool f0 = v0 >= 0.0f, f1 = v1 >= 0.0f, f2 = v2 >= 0.0f, f3 = v3 >= 0.0f;
         const float2 na = make_float2(__fmul_rn(dt, -fabsf(v0)), __fmul_rn(dt, -fabsf(v1)));
         const float2 nb = make_float2(__fmul_rn(dt, -fabsf(v2)), __fmul_rn(dt, -fabsf(v3)));
@@ -256,7 +253,7 @@ struct Prop {
     __device__ __forceinline__ static void ystep(const Ctx& c, float dt, const Row& prev, const Row& cur,
                                                  const Row& next, Row& o) {
         const Q &m = prev.q[CV], &p = next.q[CV];
-        const float v0 = dom(m.a.x, p.a.x), v1 = dom(m.a.y, p.a.y), v2 = dom(m.b.x, p.b.x), v3 = dom(m.b.y, p.b.y);
+        const float v0 = dominant(m.a.x, p.a.x), v1 = dominant(m.a.y, p.a.y), v2 = dominant(m.b.x, p.b.x), v3 = dominant(m.b.y, p.b.y);
         const bool f0 = v0 >= 0.0f, f1 = v1 >= 0.0f, f2 = v2 >= 0.0f, f3 = v3 >= 0.0f;
         const float2 na = make_float2(__fmul_rn(dt, -fabsf(v0)), __fmul_rn(dt, -fabsf(v1)));
         const float2 nb = make_float2(__fmul_rn(dt, -fabsf(v2)), __fmul_rn(dt, -fabsf(v3)));
