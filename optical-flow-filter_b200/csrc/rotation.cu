@@ -5,11 +5,11 @@
 // include/flowfilter/gpu/device/propagation_k.h:49-132).
 //
 // The reference runs 2N launches (a Y pass then an X pass per iteration, each a full-image
-// round trip through HBM or L2).  Here one CTA computes one 32 x 32 output tile: it loads the
-// image over the tile plus a halo of P pixels (P = iterations in this launch) into shared
-// memory with the flow, then runs all 2P passes there, each over a region one pixel smaller
-// along its axis (clamped at the image edges as the reference's texture reads are), and
-// writes only the tile.  More than kMaxFused iterations take several launches through a
+// round trip through HBM or L2).  Here one CTA computes a band of rows of a 64-column window: it
+// loads the image over them plus a halo of P pixels (P = iterations in this launch) into shared
+// memory with the flow, then runs all P iterations there, each over a region one pixel smaller
+// (clamped at the image edges as the reference's texture reads are), and writes only its own
+// pixels.  More than kMaxFused iterations take several launches through a
 // caller workspace.  The rotational flow is computed in the same kernel from the camera and
 // the angular velocity (and written once), so the predictor is one launch.
 //
@@ -47,13 +47,12 @@ struct LWArgs {
     size_t src_pitch;
     float* dst;
     size_t dst_pitch;
-    int H, W, passes, tile;
+    int H, W, passes;
     float dt;
 };
 
-__device__ __forceinline__ float2 rotational_flow(const LWArgs& a, int x, int y) {
-    const float px = __fdiv_rn(__fsub_rn((float)x, a.cx), a.ax);
-    const float py = __fdiv_rn(__fsub_rn((float)y, a.cy), a.ay);
+// px, py: the pixel on the unit image plane
+__device__ __forceinline__ float2 rotational_flow(const LWArgs& a, int x, int y, float px, float py) {
     const float c_x = __fmaf_rn(-a.wz, py, a.wy);
     const float c_y = __fmaf_rn(a.wz, px, -a.wx);
     const float c_z = __fmaf_rn(a.wx, py, -__fmul_rn(a.wy, px));
@@ -82,117 +81,168 @@ __device__ __forceinline__ float lw4(float m, float i0, float p, float b, float 
     return __fmaf_rn(d2, b2, __fmaf_rn(-d0, b, i0));
 }
 
+// two adjacent pixels of D channels
 template <int D>
-struct Pix {
-    float v[D];
+struct Pix2 {
+    float a[D], b[D];
 };
 
-// One CTA: the tile [tx0, tx0 + T) x [ty0, ty0 + T) of the output after `passes` iterations.
-// Shared memory: flow (float2) and two D-float buffers over the region
-// [rx0, rx1) x [ry0, ry1) = the tile grown by `passes` and cut to the image.
+// rows of 64 columns in shared memory, two pixels per lane: the image, then dt times the flow
+constexpr int kCols = 64, kWarps = 8;
+__host__ __device__ constexpr int row_bytes(int D) { return kCols * 4 * D + kCols * 8; }
+// halo columns of a window (lanes hold even pairs) and the columns from a window to the next
+__host__ __device__ constexpr int halo_of(int passes) { return (passes + 1) & ~1; }
+__host__ __device__ constexpr int step_of(int passes) { return kCols - 2 * halo_of(passes); }
+
+template <int D>
+__device__ __forceinline__ Pix2<D> lds(const char* row, int lane) {
+    Pix2<D> v;
+    if constexpr (D == 1) {
+        const float2 q = reinterpret_cast<const float2*>(row)[lane];
+        v.a[0] = q.x, v.b[0] = q.y;
+    } else {
+        const float4 q = reinterpret_cast<const float4*>(row)[2 * lane], r = reinterpret_cast<const float4*>(row)[2 * lane + 1];
+        v.a[0] = q.x, v.a[1] = q.y, v.a[2] = q.z, v.a[3] = q.w;
+        v.b[0] = r.x, v.b[1] = r.y, v.b[2] = r.z, v.b[3] = r.w;
+    }
+    return v;
+}
+template <int D>
+__device__ __forceinline__ void sts(char* row, int lane, const Pix2<D>& v) {
+    if constexpr (D == 1) {
+        reinterpret_cast<float2*>(row)[lane] = make_float2(v.a[0], v.b[0]);
+    } else {
+        reinterpret_cast<float4*>(row)[2 * lane] = make_float4(v.a[0], v.a[1], v.a[2], v.a[3]);
+        reinterpret_cast<float4*>(row)[2 * lane + 1] = make_float4(v.b[0], v.b[1], v.b[2], v.b[3]);
+    }
+}
+// one update of a pixel from its neighbours along AXIS
+template <int D, int AXIS>
+__device__ __forceinline__ void update(const float (&m)[D], const float (&i0)[D], const float (&p)[D], float R,
+                                       float (&o)[D]) {
+    if constexpr (D == 1) {
+        o[0] = lw1<AXIS>(m[0], i0[0], p[0], R);
+    } else {
+        // R / 2 and R^2 / 2 as the reference rounds them from double: the halving is exact, so
+        // the float products round the same values (where R / 2 underflows, R^2 / 2 is zero)
+        const float b = __fmul_rn(0.5f, R), b2 = __fmul_rn(b, R);
+#pragma unroll
+        for (int ch = 0; ch < D; ++ch) o[ch] = lw4(m[ch], i0[ch], p[ch], b, b2);
+    }
+}
+
+// One CTA: a window of 64 columns (two per lane) and `rows` output rows.  The image and dt times
+// the flow over the rows and P more on each side go to shared memory once; a pass then gives
+// every warp a run of rows, of which it makes the Y update from a three-row register window and,
+// from the lanes beside it, the X update, and stores the row in place: one pass over shared
+// memory and two barriers per iteration.  The outer P columns of a window belong to its
+// neighbours.  Bound by the latency of the depth-1 update's conversions and FP64 chain.
+// Measured (us, launches back to back, with the rotational flow), against 32x32 tiles whose X and
+// Y updates were passes of their own over 32-lane steps of a 40-column region: 640x480 depth 1,
+// 4 iterations 8.2 against 19.8; depth 4 9.8 against 24.9; 1920x1080 depth 1 36.5 against 75.5;
+// 2048x2048 depth 4, 16 iterations 616 against 1668.
 template <int D, bool ROT>
-__global__ void __launch_bounds__(256) lw_tile_k(LWArgs a) {
+__global__ void __launch_bounds__(32 * kWarps) lw_rows_k(LWArgs a, int nwx, int rows) {
     grid_dep_wait();
-    extern __shared__ __align__(16) unsigned char smem[];
-    const int T = a.tile, P = a.passes, H = a.H, W = a.W;
-    const int tx0 = blockIdx.x * T, ty0 = blockIdx.y * T;
-    const int rx0 = max(tx0 - P, 0), ry0 = max(ty0 - P, 0);
-    const int rx1 = min(tx0 + T + P, W), ry1 = min(ty0 + T + P, H);
-    const int RW = rx1 - rx0, RH = ry1 - ry0;
-    float2* fl = reinterpret_cast<float2*>(smem);
-    Pix<D>* A = reinterpret_cast<Pix<D>*>(fl + (size_t)RW * RH);
-    Pix<D>* B = A + (size_t)RW * RH;
-    const int lx = threadIdx.x, ly = threadIdx.y;  // 32 x 8
-    // load the image and the flow over the region
-    for (int y = ry0 + ly; y < ry1; y += 8) {
+    extern __shared__ __align__(16) char smem[];
+    constexpr int ROWB = row_bytes(D), IMG = kCols * 4 * D;
+    const int P = a.passes, H = a.H, W = a.W;
+    const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
+    const int wx = blockIdx.x % nwx, ys = blockIdx.x / nwx * rows, ye = min(ys + rows, H);
+    const int x0 = wx * step_of(P), c0 = x0 + 2 * lane;
+    const int xo = wx == 0 ? 0 : x0 + halo_of(P), xe = wx == nwx - 1 ? W : x0 + kCols - halo_of(P);
+    const int nout = c0 >= xo && c0 < xe ? min(2, W - c0) : 0;  // pixels this lane stores
+    const int ca = min(c0, W - 1), cb = min(c0 + 1, W - 1);
+    const bool e_l = c0 == 0, e_ra = c0 == W - 1, e_rb = c0 + 1 == W - 1;
+    const int sy0 = max(ys - P, 0), sy1 = min(ye + P, H);
+    // image and dt * flow of the rows
+    float pxa = 0.f, pxb = 0.f;
+    if (ROT) {
+        pxa = __fdiv_rn(__fsub_rn((float)ca, a.cx), a.ax);
+        pxb = __fdiv_rn(__fsub_rn((float)cb, a.cx), a.ax);
+    }
+    for (int y = sy0 + warp; y < sy1; y += kWarps) {
+        char* row = smem + (y - sy0) * ROWB;
         const float* srow = reinterpret_cast<const float*>(reinterpret_cast<const char*>(a.src) + y * a.src_pitch);
-        for (int x = rx0 + lx; x < rx1; x += 32) {
-            const int k = (y - ry0) * RW + (x - rx0);
-            Pix<D> px;
-            if constexpr (D == 4) {
-                const float4 q = reinterpret_cast<const float4*>(srow)[x];
-                px.v[0] = q.x;
-                px.v[1] = q.y;
-                px.v[2] = q.z;
-                px.v[3] = q.w;
-            } else {
-                px.v[0] = srow[x];
-            }
-            A[k] = px;
-            float2 f;
-            if (ROT) {
-                f = rotational_flow(a, x, y);
-                if (x >= tx0 && x < tx0 + T && y >= ty0 && y < ty0 + T)
-                    reinterpret_cast<float2*>(reinterpret_cast<char*>(a.flow_out) + y * a.flow_out_pitch)[x] = f;
-            } else {
-                f = reinterpret_cast<const float2*>(reinterpret_cast<const char*>(a.flow) + y * a.flow_pitch)[x];
-            }
-            fl[k] = f;
+        Pix2<D> v;
+        if constexpr (D == 4) {
+            const float4 q = __ldg(reinterpret_cast<const float4*>(srow) + ca), r = __ldg(reinterpret_cast<const float4*>(srow) + cb);
+            v.a[0] = q.x, v.a[1] = q.y, v.a[2] = q.z, v.a[3] = q.w;
+            v.b[0] = r.x, v.b[1] = r.y, v.b[2] = r.z, v.b[3] = r.w;
+        } else {
+            v.a[0] = __ldg(srow + ca);
+            v.b[0] = __ldg(srow + cb);
         }
+        float2 fa, fb;
+        if (ROT) {
+            const float py = __fdiv_rn(__fsub_rn((float)y, a.cy), a.ay);
+            fa = rotational_flow(a, ca, y, pxa, py);
+            fb = rotational_flow(a, cb, y, pxb, py);
+            if (y >= ys && y < ye) {
+                float2* frow = reinterpret_cast<float2*>(reinterpret_cast<char*>(a.flow_out) + y * a.flow_out_pitch);
+                if (nout > 0) frow[c0] = fa;
+                if (nout > 1) frow[c0 + 1] = fb;
+            }
+        } else {
+            const float2* frow = reinterpret_cast<const float2*>(reinterpret_cast<const char*>(a.flow) + y * a.flow_pitch);
+            fa = __ldg(frow + ca);
+            fb = __ldg(frow + cb);
+        }
+        sts<D>(row, lane, v);
+        reinterpret_cast<float4*>(row + IMG)[lane] = make_float4(__fmul_rn(a.dt, fa.x), __fmul_rn(a.dt, fa.y),
+                                                                 __fmul_rn(a.dt, fb.x), __fmul_rn(a.dt, fb.y));
     }
     grid_dep_launch();
     __syncthreads();
-    // valid region of the current buffer; a pass keeps the rows (columns) whose neighbours
-    // are valid, the image edges clamping to themselves
-    int vx0 = rx0, vx1 = rx1, vy0 = ry0, vy1 = ry1;
-    const float dt = a.dt;
-    for (int it = 0; it < P; ++it) {
-        // Y pass, A -> B
-        vy0 = vy0 == 0 ? 0 : vy0 + 1;
-        vy1 = vy1 == H ? H : vy1 - 1;
-        for (int y = vy0 + ly; y < vy1; y += 8) {
-            const int rm = (max(y - 1, 0) - ry0) * RW, r0 = (y - ry0) * RW, rp = (min(y + 1, H - 1) - ry0) * RW;
-            for (int x = vx0 + lx; x < vx1; x += 32) {
-                const int c = x - rx0;
-                const float R = __fmul_rn(dt, fl[r0 + c].y);
-                const Pix<D> m = A[rm + c], i0 = A[r0 + c], p = A[rp + c];
-                Pix<D> o;
-                if constexpr (D == 1) {
-                    o.v[0] = lw1<1>(m.v[0], i0.v[0], p.v[0], R);
-                } else {
-                    const float b = __double2float_rn(__dmul_rn(0.5, (double)R));
-                    const float b2 = __double2float_rn(__dmul_rn(__dmul_rn(0.5, (double)R), (double)R));
+    for (int it = 1; it <= P; ++it) {
+        // rows the later iterations need, a run of them per warp
+        const int r = P - it, ya = max(ys - r, 0), n = min(ye + r, H) - ya;
+        const int y0 = ya + n * warp / kWarps, y1 = ya + n * (warp + 1) / kWarps;
+        // the rows around the run belong to other warps, which overwrite them: read first (at an
+        // image edge the row itself is its neighbour)
+        Pix2<D> prev, last;
+        if (y0 < y1) {
+            prev = lds<D>(smem + (max(y0 - 1, 0) - sy0) * ROWB, lane);
+            last = lds<D>(smem + (min(y1, H - 1) - sy0) * ROWB, lane);
+        }
+        __syncthreads();
+        if (y0 < y1) {
+            Pix2<D> cur = lds<D>(smem + (y0 - sy0) * ROWB, lane);
+#pragma unroll 2
+            for (int y = y0; y < y1; ++y) {
+                char* row = smem + (y - sy0) * ROWB;
+                const Pix2<D> next = y + 1 < y1 ? lds<D>(row + ROWB, lane) : last;
+                const float4 R = reinterpret_cast<const float4*>(row + IMG)[lane];  // (x, y) of both pixels
+                Pix2<D> t, o;
+                update<D, 1>(prev.a, cur.a, next.a, R.y, t.a);
+                update<D, 1>(prev.b, cur.b, next.b, R.w, t.b);
+                float ma[D], pa[D], pb[D];
 #pragma unroll
-                    for (int ch = 0; ch < D; ++ch) o.v[ch] = lw4(m.v[ch], i0.v[ch], p.v[ch], b, b2);
+                for (int ch = 0; ch < D; ++ch) {
+                    const float l = __shfl_up_sync(0xffffffffu, t.b[ch], 1), rr = __shfl_down_sync(0xffffffffu, t.a[ch], 1);
+                    ma[ch] = e_l ? t.a[ch] : l;
+                    pa[ch] = e_ra ? t.a[ch] : t.b[ch];
+                    pb[ch] = e_rb ? t.b[ch] : rr;
                 }
-                B[r0 + c] = o;
+                update<D, 0>(ma, t.a, pa, R.x, o.a);
+                update<D, 0>(t.a, t.b, pb, R.z, o.b);
+                if (it < P) {
+                    sts<D>(row, lane, o);
+                } else {
+                    float* drow = reinterpret_cast<float*>(reinterpret_cast<char*>(a.dst) + y * a.dst_pitch);
+                    if constexpr (D == 4) {
+                        if (nout > 0) reinterpret_cast<float4*>(drow)[c0] = make_float4(o.a[0], o.a[1], o.a[2], o.a[3]);
+                        if (nout > 1) reinterpret_cast<float4*>(drow)[c0 + 1] = make_float4(o.b[0], o.b[1], o.b[2], o.b[3]);
+                    } else {
+                        if (nout > 0) drow[c0] = o.a[0];
+                        if (nout > 1) drow[c0 + 1] = o.b[0];
+                    }
+                }
+                prev = cur;
+                cur = next;
             }
         }
         __syncthreads();
-        // X pass, B -> A
-        vx0 = vx0 == 0 ? 0 : vx0 + 1;
-        vx1 = vx1 == W ? W : vx1 - 1;
-        for (int y = vy0 + ly; y < vy1; y += 8) {
-            const int r0 = (y - ry0) * RW;
-            for (int x = vx0 + lx; x < vx1; x += 32) {
-                const int cm = max(x - 1, 0) - rx0, c = x - rx0, cp = min(x + 1, W - 1) - rx0;
-                const float R = __fmul_rn(dt, fl[r0 + c].x);
-                const Pix<D> m = B[r0 + cm], i0 = B[r0 + c], p = B[r0 + cp];
-                Pix<D> o;
-                if constexpr (D == 1) {
-                    o.v[0] = lw1<0>(m.v[0], i0.v[0], p.v[0], R);
-                } else {
-                    const float b = __double2float_rn(__dmul_rn(0.5, (double)R));
-                    const float b2 = __double2float_rn(__dmul_rn(__dmul_rn(0.5, (double)R), (double)R));
-#pragma unroll
-                    for (int ch = 0; ch < D; ++ch) o.v[ch] = lw4(m.v[ch], i0.v[ch], p.v[ch], b, b2);
-                }
-                A[r0 + c] = o;
-            }
-        }
-        __syncthreads();
-    }
-    // the tile
-    const int ox1 = min(tx0 + T, W), oy1 = min(ty0 + T, H);
-    for (int y = ty0 + ly; y < oy1; y += 8) {
-        float* drow = reinterpret_cast<float*>(reinterpret_cast<char*>(a.dst) + y * a.dst_pitch);
-        for (int x = tx0 + lx; x < ox1; x += 32) {
-            const Pix<D> o = A[(y - ry0) * RW + (x - rx0)];
-            if constexpr (D == 4)
-                reinterpret_cast<float4*>(drow)[x] = make_float4(o.v[0], o.v[1], o.v[2], o.v[3]);
-            else
-                drow[x] = o.v[0];
-        }
     }
 }
 
@@ -201,39 +251,34 @@ __global__ void rotational_flow_k(LWArgs a) {
     grid_dep_launch();
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
     if (x >= a.W || y >= a.H) return;
-    reinterpret_cast<float2*>(reinterpret_cast<char*>(a.flow_out) + y * a.flow_out_pitch)[x] = rotational_flow(a, x, y);
-}
-
-// 32 x 32 tiles: a VGA image gives 300 CTAs, several resident per SM (each a few to 164 KB
-// of shared memory), which hides the shared-memory and FP64 latency of the passes
-int tile_of(int D, int passes) {
-    (void)D;
-    (void)passes;
-    return 32;
-}
-
-size_t smem_of(int D, int tile, int passes) {
-    const size_t r = (size_t)(tile + 2 * passes);
-    return r * r * (8 + 2 * 4 * (size_t)D);
+    reinterpret_cast<float2*>(reinterpret_cast<char*>(a.flow_out) + y * a.flow_out_pitch)[x] =
+        rotational_flow(a, x, y, __fdiv_rn(__fsub_rn((float)x, a.cx), a.ax), __fdiv_rn(__fsub_rn((float)y, a.cy), a.ay));
 }
 
 template <int D, bool ROT>
 cudaError_t launch_lw(LWArgs a, cudaStream_t s) {
-    const size_t smem = smem_of(D, a.tile, a.passes);
-    // once per device: room for the largest launch (kMaxFused iterations); no static smem
-    static std::atomic<unsigned long long> prepared{0};
-    int dev = 0;
+    const int step = step_of(a.passes);
+    const int nwx = 1 + (std::max(a.W - kCols, 0) + step - 1) / step;
+    int dev = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    // Bands of as few rows as give two windows per SM (16 rows at the least, against halo rows;
+    // at the most what two blocks' shared memory holds)
+    const int most = 108 * 1024 / row_bytes(D) - 2 * a.passes;
+    const int bands = std::max(1, 2 * std::max(sms, 1) / nwx);
+    const int rows = std::min(std::min(std::max((a.H + bands - 1) / bands, 16), most), a.H);
+    const size_t smem = (size_t)(rows + 2 * a.passes) * row_bytes(D);
+    // once per device: room for the largest launch; no static smem
+    static std::atomic<unsigned long long> prepared{0};
     const unsigned long long bit = 1ull << (dev & 63);
     if (!(prepared.load() & bit)) {
-        e = cudaFuncSetAttribute(lw_tile_k<D, ROT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem_of(D, tile_of(D, kMaxFused), kMaxFused));
+        e = cudaFuncSetAttribute(lw_rows_k<D, ROT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 108 * 1024);
         if (e != cudaSuccess) return e;
         prepared.fetch_or(bit);
     }
-    const dim3 grid((a.W + a.tile - 1) / a.tile, (a.H + a.tile - 1) / a.tile);
-    return launch_k(lw_tile_k<D, ROT>, grid, dim3(32, 8), smem, s, a);
+    const long blocks = (long)nwx * ((a.H + rows - 1) / rows);
+    return launch_k(lw_rows_k<D, ROT>, dim3((unsigned)blocks), dim3(32 * kWarps), smem, s, a, nwx, rows);
 }
 
 // Full propagation: ceil(n / kMaxFused) launches ending in `out`; earlier ones alternate
@@ -250,7 +295,6 @@ cudaError_t propagate(LWArgs a, int depth, int iterations, bool rot, float* out,
         a.dst = to_out ? out : ws;
         a.dst_pitch = to_out ? out_pitch : ws_pitch;
         a.passes = p;
-        a.tile = tile_of(depth, p);
         const bool r = rot && i == 0;
         cudaError_t e;
         if (depth == 1)
