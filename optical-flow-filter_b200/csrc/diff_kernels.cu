@@ -848,138 +848,282 @@ __global__ void __launch_bounds__(256) smooth_iter_bwd_k(const T* __restrict__ w
     block_sum<T, 5>(gw, part + 5 * block_linear(), false);
 }
 
-// asynchronous global -> shared copy of N bytes (4, 8 or 16; both addresses N-aligned)
-template <int N>
-__device__ __forceinline__ void cp_async(void* dst, const void* src) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(d), "l"(src), "n"(N) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() {
-    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
-}
-
-// Adjoint of one propagation iteration (X sub-step, then Y sub-step) of a 32 x 32 tile in one
-// block of the frame driver.  Staged in shared memory in one batch of asynchronous copies:
-// the gradient of the Y sub-step's output on the tile and one halo row and column, the Y
-// sub-step's input on the tile's columns plus one and the rows plus two each side, the X
-// sub-step's input on the tile's rows and the columns plus two each side (the tape, or the
-// state before the first sub-step).  Then the Y adjoint on the tile's rows and the halo
-// columns (shared), and the X adjoint from it into the X sub-step's input gradient (stored,
-// or added when ACC).  Entries outside the image are never read.
-constexpr int kPG = kST + 2;
-constexpr int kPropThreads = 512;  // 32 x 16
+// Rows of a propagated field, N adjacent pixels per lane: float takes two, so that a row of a
+// window is one vector access per part where the alignment allows (vec), double one.
+template <typename T>
+constexpr int kPropPix = sizeof(T) == 4 ? 2 : 1;
+constexpr int kPropWarps = 4;
+constexpr int kPropRunWarps = 12;  // resident warps per multiprocessor that a launch aims at (160 registers)
+template <typename T>
+constexpr int prop_cols() { return 32 * kPropPix<T>; }
+// an output column's gradient needs the fields two columns away: the outer two of a window
+// belong to its neighbours
+template <typename T>
+constexpr int prop_step() { return prop_cols<T>() - 4; }
 template <typename T, bool PAYLOAD>
-struct PropTile {
-    using V = typename Pair<T>::V;
-    static constexpr int NC = PAYLOAD ? 5 : 2;
-    // pixel fields of a staged region: f pairs [, s, v pairs]
-    template <int R, int C>
-    struct Field {
-        V f[R][C];
-        T s[PAYLOAD ? R : 1][PAYLOAD ? C : 1];
-        V v[PAYLOAD ? R : 1][PAYLOAD ? C : 1];
-    };
-    Field<kPG, kPG> go;      // output gradient: rows y0-1.., cols x0-1..
-    Field<kST + 4, kPG> ty;  // Y sub-step input: rows y0-2.., cols x0-1..
-    Field<kST, kST + 4> tx;  // X sub-step input: rows y0.., cols x0-2..
-    T mid[NC][kST][kPG];     // gradient of the X sub-step's output: rows y0.., cols x0-1..
-};
-
-// copy pixel k of a field into slot (r, c) of a staged region
-template <typename T, bool PAYLOAD, typename F>
-__device__ __forceinline__ void stage_px(F& dst, int r, int c, const T* f, const T* s, const T* v, size_t k) {
-    constexpr int P = 2 * sizeof(T);
-    if (f) {
-        cp_async<P>(&dst.f[r][c], f + 2 * k);
-    } else {  // an absent gradient: zeros
-        dst.f[r][c].x = T(0);
-        dst.f[r][c].y = T(0);
+struct PropRow {
+    static constexpr int N = kPropPix<T>, NC = PAYLOAD ? 5 : 2;
+    T c[N][NC];
+    // pixel k and, with N = 2, k1; an absent f reads as zero
+    __device__ __forceinline__ void load(const T* f, const T* s, const T* v, size_t k, size_t k1, bool vec) {
+        if constexpr (N == 2) {
+            if (vec) {
+                const float4 q = f ? *reinterpret_cast<const float4*>(f + 2 * k) : make_float4(0.f, 0.f, 0.f, 0.f);
+                c[0][0] = q.x, c[0][1] = q.y, c[1][0] = q.z, c[1][1] = q.w;
+                if constexpr (PAYLOAD) {
+                    const float2 r = *reinterpret_cast<const float2*>(s + k);
+                    const float4 t = *reinterpret_cast<const float4*>(v + 2 * k);
+                    c[0][2] = r.x, c[1][2] = r.y;
+                    c[0][3] = t.x, c[0][4] = t.y, c[1][3] = t.z, c[1][4] = t.w;
+                }
+                return;
+            }
+            px(f, s, v, k1, c[1]);
+        }
+        px(f, s, v, k, c[0]);
     }
-    if constexpr (PAYLOAD) {
-        cp_async<sizeof(T)>(&dst.s[r][c], s + k);
-        cp_async<P>(&dst.v[r][c], v + 2 * k);
-    }
-}
-template <typename T, bool PAYLOAD, typename F>
-__device__ __forceinline__ void read_px(const F& src, int r, int c, T (&o)[PAYLOAD ? 5 : 2]) {
-    o[0] = src.f[r][c].x;
-    o[1] = src.f[r][c].y;
-    if constexpr (PAYLOAD) {
-        o[2] = src.s[r][c];
-        o[3] = src.v[r][c].x;
-        o[4] = src.v[r][c].y;
-    }
-}
-
-template <typename T, bool PAYLOAD, bool ACC>
-__global__ void __launch_bounds__(kPropThreads) prop_iter_bwd_k(const T* __restrict__ xf, const T* __restrict__ xs,
-                                                                const T* __restrict__ xv, const T* __restrict__ yf,
-                                                                const T* __restrict__ ys, const T* __restrict__ yv,
-                                                                const T* __restrict__ gfo, const T* __restrict__ gso,
-                                                                const T* __restrict__ gvo, T* __restrict__ gf,
-                                                                T* __restrict__ gs, T* __restrict__ gv, int H, int W,
-                                                                T dt, int border) {
-    grid_dep_wait();
-    using Tile = PropTile<T, PAYLOAD>;
-    constexpr int NC = Tile::NC;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    Tile& S = *reinterpret_cast<Tile*>(smem_raw);
-    const int tid = threadIdx.y * blockDim.x + threadIdx.x;
-    const int x0 = blockIdx.x * kST, y0 = blockIdx.y * kST;
-    const size_t base = (size_t)blockIdx.z * H * W;
-    for (int e = tid; e < kPG * kPG; e += kPropThreads) {
-        const int r = e / kPG, c = e - r * kPG, y = y0 - 1 + r, x = x0 - 1 + c;
-        if (y >= 0 && y < H && x >= 0 && x < W)
-            stage_px<T, PAYLOAD>(S.go, r, c, gfo, gso, gvo, base + (size_t)y * W + x);
-    }
-    for (int e = tid; e < (kST + 4) * kPG; e += kPropThreads) {
-        const int r = e / kPG, c = e - r * kPG, y = y0 - 2 + r, x = x0 - 1 + c;
-        if (y >= 0 && y < H && x >= 0 && x < W) stage_px<T, PAYLOAD>(S.ty, r, c, yf, ys, yv, base + (size_t)y * W + x);
-    }
-    for (int e = tid; e < kST * (kST + 4); e += kPropThreads) {
-        const int r = e / (kST + 4), c = e - r * (kST + 4), y = y0 + r, x = x0 - 2 + c;
-        if (y < H && x >= 0 && x < W) stage_px<T, PAYLOAD>(S.tx, r, c, xf, xs, xv, base + (size_t)y * W + x);
-    }
-    cp_async_wait_all();
-    __syncthreads();
-    // Y adjoint at rows y0.., columns x0-1..
-    for (int e = tid; e < kST * kPG; e += kPropThreads) {
-        const int r = e / kPG, c = e - r * kPG;
-        const int y = y0 + r, x = x0 - 1 + c;
-        if (y >= H || x < 0 || x >= W) continue;
-        T acc[NC];
-        prop_adj_at<T, 1, PAYLOAD>(
-            y, H, x >= border && x < W - border, border, dt,
-            [&](int p, T(&o)[NC]) { read_px<T, PAYLOAD>(S.ty, p - y0 + 2, c, o); },
-            [&](int p, T(&o)[NC]) { read_px<T, PAYLOAD>(S.go, p - y0 + 1, c, o); }, acc);
-#pragma unroll
-        for (int ch = 0; ch < NC; ++ch) S.mid[ch][r][c] = acc[ch];
-    }
-    __syncthreads();
-    grid_dep_launch();  // the next kernel's blocks may now take this block's place
-    // X adjoint at the tile's pixels
-    for (int e = tid; e < kST * kST; e += kPropThreads) {
-        const int r = e / kST, c = e - r * kST;
-        const int y = y0 + r, x = x0 + c;
-        if (y >= H || x >= W) continue;
-        T acc[NC];
-        prop_adj_at<T, 0, PAYLOAD>(
-            x, W, y >= border && y < H - border, border, dt,
-            [&](int p, T(&o)[NC]) { read_px<T, PAYLOAD>(S.tx, r, p - x0 + 2, o); },
-            [&](int p, T(&o)[NC]) {
-#pragma unroll
-                for (int ch = 0; ch < NC; ++ch) o[ch] = S.mid[ch][r][p - x0 + 1];
-            },
-            acc);
-        const size_t k = base + (size_t)y * W + x;
-        put<ACC>(gf[2 * k], acc[0]);
-        put<ACC>(gf[2 * k + 1], acc[1]);
+    __device__ __forceinline__ static void px(const T* f, const T* s, const T* v, size_t k, T (&o)[NC]) {
+        using V = typename Pair<T>::V;
+        o[0] = o[1] = T(0);
+        if (f) {
+            const V q = reinterpret_cast<const V*>(f)[k];
+            o[0] = q.x, o[1] = q.y;
+        }
         if constexpr (PAYLOAD) {
-            put<ACC>(gs[k], acc[2]);
-            put<ACC>(gv[2 * k], acc[3]);
-            put<ACC>(gv[2 * k + 1], acc[4]);
+            const V t = reinterpret_cast<const V*>(v)[k];
+            o[2] = s[k], o[3] = t.x, o[4] = t.y;
         }
     }
+};
+
+// What one output i of an upwind sub-step hands to the gradients of its stencil: the weights of
+// its own gradient at i and at the neighbours i-1 (lo) and i+1 (hi), and the gradient of the
+// dominant velocity, which goes to the neighbour it was taken from.
+template <typename T, int NC>
+struct UpwindAdj {
+    T self, lo, hi, gdv;
+    bool in, pos, take_p;
+    // g: output gradient; dm, dp: backward and forward differences; vm, vp: the axis' velocity
+    // at the neighbours
+    __device__ __forceinline__ void make(const T (&g)[NC], const T (&dm)[NC], const T (&dp)[NC], T vm, T vp, bool in_,
+                                         T dt) {
+        in = in_;
+        take_p = fabs(vp) > fabs(vm);
+        const T dv = take_p ? vp : vm;
+        const T t = dt * dv;
+        pos = dv >= T(0);
+        const T dtq = in ? dt : T(0);
+        self = in ? (pos ? T(1) - t : T(1) + t) : T(1);  // a frozen output passes its gradient
+        lo = in && pos ? t : T(0);
+        hi = in && !pos ? -t : T(0);
+        gdv = T(0);
+#pragma unroll
+        for (int c = 0; c < NC; ++c) gdv -= g[c] * dtq * (pos ? dm[c] : dp[c]);
+    }
+    // clamped stencils, at the ends of the line, hand their neighbour's share to themselves
+    __device__ __forceinline__ void clamped(const T (&g)[NC], bool first, bool last, T& axis, T (&acc)[NC]) const {
+        if (!in) return;
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            if (first) acc[c] += g[c] * lo;
+            if (last) acc[c] += g[c] * hi;
+        }
+        if (first && !take_p) axis += gdv;
+        if (last && take_p) axis += gdv;
+    }
+};
+
+// Adjoint of one propagation iteration (X sub-step, then Y sub-step) of the frame driver, by
+// independent warps: a warp takes a window of columns and a run of rows and walks down it.  Row
+// i's Y outputs hand their shares to the gradients of rows i-1, i and i+1, kept in registers;
+// row i-1 is then complete, and its X sub-step follows in the next step, beside row i+1's Y
+// outputs, from the lanes beside each pixel.  The values a row needs are loaded a step ahead; no
+// shared memory, no barrier.  CLAMP: the border may be 0, so that live stencils clamp.  Sums run in the
+// order of the output positions, as in prop_adj_at.
+// Bound by issue and the latency of a row's chain (three warps per scheduler at 160 registers).
+// Measured, 16 images of 256x256 with payload: 24.5 us, 27.5 us adding to the caller's
+// gradient, against 32.2 and 40.9 us for a 32 x 32 tile that staged every region in shared
+// memory and formed each output's shares three times, at every pixel that collects them.  One
+// pixel per lane and more warps: 27.8 and 30.3 us.
+template <typename T, bool PAYLOAD, bool ACC, bool CLAMP>
+__global__ void __launch_bounds__(32 * kPropWarps)
+    prop_iter_bwd_k(const T* __restrict__ xf, const T* __restrict__ xs, const T* __restrict__ xv,
+                    const T* __restrict__ yf, const T* __restrict__ ys, const T* __restrict__ yv,
+                    const T* __restrict__ gfo, const T* __restrict__ gso, const T* __restrict__ gvo,
+                    T* __restrict__ gf, T* __restrict__ gs, T* __restrict__ gv, int H, int W, T dt, int border, int nwx,
+                    int bands, int rows, int warps, bool vec) {
+    using R = PropRow<T, PAYLOAD>;
+    constexpr int N = R::N, NC = R::NC;
+    constexpr unsigned kAll = 0xffffffffu;
+    grid_dep_wait();
+    const int lane = threadIdx.x & 31;
+    const int id = blockIdx.x * kPropWarps + __shfl_sync(kAll, (int)(threadIdx.x >> 5), 0);
+    if (id >= warps) return;
+    const int wx = id % nwx, rest = id / nwx;
+    const int r0 = rest % bands * rows, r1 = min(r0 + rows, H);
+    const size_t base = (size_t)(rest / bands) * H * W;
+    const int x0 = wx * prop_step<T>(), c0 = x0 + N * lane;
+    const int xo = wx == 0 ? 0 : x0 + 2, xe = wx == nwx - 1 ? W : x0 + prop_cols<T>() - 2;  // columns stored
+    // columns read (with vec, W is even: both or neither pixel of a lane inside)
+    const int ca = vec ? min(c0, W - 2) : min(c0, W - 1), cb = min(c0 + N - 1, W - 1);
+    auto load = [&](R& r, const T* f, const T* s, const T* v, int y) {
+        const size_t row = base + (size_t)y * W;
+        r.load(f, s, v, row + ca, row + cb, vec);
+    };
+    bool xin[N];
+#pragma unroll
+    for (int n = 0; n < N; ++n) xin[n] = c0 + n >= border && c0 + n < W - border;
+
+    R cur, nxt, g, tx;       // Y sub-step input rows i, i+1; output gradient of row i; X input of row i-2
+    T dm[N][NC], vm[N];      // row i minus row i-1; row i-1's y velocity
+    T up[N][NC], at[N][NC];  // gradients collected for rows i-1, i
+    T fin[N][NC];            // the complete gradient of row i-2
+    const int i0 = max(r0 - 1, 0);
+    {
+        R prev;
+        load(prev, yf, ys, yv, max(i0 - 1, 0));
+        load(cur, yf, ys, yv, i0);
+        load(nxt, yf, ys, yv, min(i0 + 1, H - 1));
+        load(g, gfo, gso, gvo, i0);
+        tx = prev;
+#pragma unroll
+        for (int n = 0; n < N; ++n) {
+            vm[n] = prev.c[n][1];
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                dm[n][c] = cur.c[n][c] - prev.c[n][c];
+                up[n][c] = at[n][c] = fin[n][c] = T(0);
+            }
+        }
+    }
+#pragma unroll 1
+    for (int i = i0; i <= r1 + 1; ++i) {
+        // the next step's rows
+        R nn, gn, txn, old;
+        load(nn, yf, ys, yv, min(i + 2, H - 1));
+        load(gn, gfo, gso, gvo, min(i + 1, H - 1));
+        load(txn, xf, xs, xv, min(max(i - 1, 0), H - 1));
+        // the X sub-step of row i-2
+        const int y = i - 2;
+        if constexpr (ACC) load(old, gf, gs, gv, min(max(y, 0), H - 1));
+        {
+            const bool row_in = y >= border && y < H - border;
+            T l[NC], r[NC];  // the pixels beside the lane's, itself at the image edges
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                const T q = __shfl_up_sync(kAll, tx.c[N - 1][c], 1);
+                l[c] = c0 == 0 ? tx.c[0][c] : q;
+                r[c] = __shfl_down_sync(kAll, tx.c[0][c], 1);
+            }
+            UpwindAdj<T, NC> u[N];
+#pragma unroll
+            for (int n = 0; n < N; ++n) {
+                T dl[NC], dr[NC], vp = T(0);
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    const T left = n == 0 ? l[c] : tx.c[0][c], self = tx.c[n][c];
+                    const T right = c0 + n == W - 1 ? self : (n == N - 1 ? r[c] : tx.c[N - 1][c]);
+                    dl[c] = self - left;
+                    dr[c] = right - self;
+                    if (c == 0) vp = right;
+                }
+                u[n].make(fin[n], dl, dr, n == 0 ? l[0] : tx.c[0][0], vp, row_in && xin[n], dt);
+            }
+            // the shares of the outputs beside the lane's pixels
+            T gl[NC], gr[NC];
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                gl[c] = __shfl_up_sync(kAll, fin[N - 1][c], 1);
+                gr[c] = __shfl_down_sync(kAll, fin[0][c], 1);
+            }
+            const T wl = __shfl_up_sync(kAll, u[N - 1].hi, 1), wr = __shfl_down_sync(kAll, u[0].lo, 1);
+            const T vl = __shfl_up_sync(kAll, u[N - 1].take_p ? u[N - 1].gdv : T(0), 1);
+            const T vr = __shfl_down_sync(kAll, u[0].take_p ? T(0) : u[0].gdv, 1);
+            const size_t row = base + (size_t)y * W;
+#pragma unroll
+            for (int n = 0; n < N; ++n) {
+                const int j = c0 + n;
+                const bool edge = j < 2 || j + 2 > W - 1;
+                const T hi = n == 0 ? wl : u[0].hi, lo = n == N - 1 ? wr : u[N - 1].lo;
+                const T gvl = n == 0 ? vl : (u[0].take_p ? u[0].gdv : T(0));
+                const T gvr = n == N - 1 ? vr : (u[N - 1].take_p ? T(0) : u[N - 1].gdv);
+                const bool in_l = row_in && j - 1 >= border && j - 1 < W - border;
+                const bool in_r = row_in && j + 1 >= border && j + 1 < W - border;
+                const bool take_l = j > 0 && (!edge || hi != T(0)), take_r = j < W - 1 && (!edge || lo != T(0));
+                T acc[NC];
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    acc[c] = T(0);
+                    if (take_l) acc[c] += (n == 0 ? gl[c] : fin[0][c]) * hi;
+                }
+                if (j > 0 && (!edge || in_l)) acc[0] += gvl;
+#pragma unroll
+                for (int c = 0; c < NC; ++c) acc[c] += fin[n][c] * u[n].self;
+                if constexpr (CLAMP) u[n].clamped(fin[n], j == 0, j == W - 1, acc[0], acc);
+#pragma unroll
+                for (int c = 0; c < NC; ++c)
+                    if (take_r) acc[c] += (n == N - 1 ? gr[c] : fin[N - 1][c]) * lo;
+                if (j < W - 1 && (!edge || in_r)) acc[0] += gvr;
+                if (y >= r0 && y < r1 && j >= xo && j < xe && j < W) {
+                    using V = typename Pair<T>::V;
+                    if constexpr (ACC) {
+#pragma unroll
+                        for (int c = 0; c < NC; ++c) acc[c] = old.c[n][c] + acc[c];
+                    }
+                    V o;
+                    o.x = acc[0], o.y = acc[1];
+                    reinterpret_cast<V*>(gf)[row + j] = o;
+                    if constexpr (PAYLOAD) {
+                        gs[row + j] = acc[2];
+                        o.x = acc[3], o.y = acc[4];
+                        reinterpret_cast<V*>(gv)[row + j] = o;
+                    }
+                }
+            }
+        }
+        // row i's Y outputs.  i = H and beyond: frozen rows at an edge, which hand nothing to row H-1
+        T dn[N][NC];
+        {
+            // rows whose sums take only the shares that reach them (their stencils clamp)
+            const bool edge_up = i - 1 < 2 || i + 1 > H - 1, edge_dn = i + 1 < 2 || i + 3 > H - 1;
+            const bool row_in = i >= border && i < H - border;
+#pragma unroll
+            for (int n = 0; n < N; ++n) {
+                T dp[NC];
+                UpwindAdj<T, NC> u;
+#pragma unroll
+                for (int c = 0; c < NC; ++c) dp[c] = nxt.c[n][c] - cur.c[n][c];
+                u.make(g.c[n], dm[n], dp, vm[n], nxt.c[n][1], row_in && xin[n], dt);
+                const bool lo = !edge_up || (u.in && u.pos), hi = !edge_dn || (u.in && !u.pos);
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    const T go = g.c[n][c];
+                    if (lo) up[n][c] += go * u.lo;
+                    at[n][c] += go * u.self;
+                    dn[n][c] = T(0);
+                    if (hi) dn[n][c] += go * u.hi;
+                    dm[n][c] = dp[c];
+                }
+                if (!edge_up || u.in) up[n][1] += u.take_p ? T(0) : u.gdv;
+                if constexpr (CLAMP) u.clamped(g.c[n], i == 0, i == H - 1, at[n][1], at[n]);
+                if (!edge_dn || u.in) dn[n][1] += u.take_p ? u.gdv : T(0);
+                vm[n] = cur.c[n][1];
+            }
+        }
+        cur = nxt;
+        nxt = nn;
+        g = gn;
+        tx = txn;
+#pragma unroll
+        for (int n = 0; n < N; ++n)
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                fin[n][c] = up[n][c];
+                up[n][c] = at[n][c];
+                at[n][c] = dn[n][c];
+            }
+    }
+    grid_dep_launch();
 }
 
 // The image model's adjoint (model_bwd1_k then model_bwd2_k) of a 32 x 32 tile in one block
@@ -1838,19 +1982,25 @@ struct Driver {
     template <bool PAYLOAD, bool ACC>
     void prop_iter_bwd(int l, const T* xf, const T* xs, const T* xv, const T* yf, const T* ys, const T* yv,
                        const T* gfo, const T* gso, const T* gvo, T* gf, T* gs, T* gv) const {
-        constexpr size_t smem = sizeof(PropTile<T, PAYLOAD>);
-        static bool prepared[64] = {};  // the dynamic shared-memory limit, set once per device
-        int dev = 0;
-        ok(cudaGetDevice(&dev));
-        if (!prepared[dev & 63]) {
-            ok(cudaFuncSetAttribute(prop_iter_bwd_k<T, PAYLOAD, ACC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)smem));
-            prepared[dev & 63] = true;
-        }
         const T dt = (T)(1.0 / g.N[l]);
-        ok(launch_k(prop_iter_bwd_k<T, PAYLOAD, ACC>, grid_tile32(g.W[l], g.H[l], g.B), dim3(32, kPropThreads / 32),
-                    smem, s, xf, xs, xv,
-                    yf, ys, yv, gfo, gso, gvo, gf, gs, gv, g.H[l], g.W[l], dt, g.border));
+        const int H = g.H[l], W = g.W[l];
+        int dev = 0, sms = 0;
+        ok(cudaGetDevice(&dev));
+        ok(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        // runs as short as fill every multiprocessor with kPropRunWarps warps, four rows at the
+        // least (a run forms the outputs of two rows beyond it)
+        const int nwx = 1 + (std::max(W - prop_cols<T>(), 0) + prop_step<T>() - 1) / prop_step<T>();
+        const long long cols = (long long)nwx * g.B, target = (long long)sms * kPropRunWarps;
+        const int rows = (int)std::min<long long>(H, std::max<long long>(4, (cols * H + target - 1) / target));
+        const int bands = (H + rows - 1) / rows;
+        const int warps = (int)(cols * bands);
+        auto a16 = [](const T* p) { return ((uintptr_t)p & 15) == 0; };
+        auto a8 = [](const T* p) { return ((uintptr_t)p & 7) == 0; };
+        const bool vec = kPropPix<T> == 2 && W % 2 == 0 && a16(xf) && a16(yf) && a16(gfo) && a8(xs) && a8(ys) &&
+                         a8(gso) && a16(xv) && a16(yv) && a16(gvo) && a16(gf) && a8(gs) && a16(gv);
+        auto kern = g.border > 0 ? prop_iter_bwd_k<T, PAYLOAD, ACC, false> : prop_iter_bwd_k<T, PAYLOAD, ACC, true>;
+        ok(launch_k(kern, dim3((warps + kPropWarps - 1) / kPropWarps), dim3(32 * kPropWarps), 0, s, xf, xs, xv, yf, ys, yv, gfo, gso, gvo, gf, gs, gv, H, W, dt, g.border,
+                    nwx, bands, rows, warps, vec));
     }
     // one smoothing iteration's adjoint (X and Y pass): input gradient stored (or added),
     // weight sums per block
