@@ -664,14 +664,21 @@ void Filter::launch_fused(int l, int band, cudaStream_t s) {
 
 // In a pyramid frame the top level's tile or slab kernel is followed on the same stream by
 // level L-2's, which reads the top's output only from its update on: the top lets it start at
-// once, and it waits only before its update (so its propagation overlaps the top level).
+// once, and it waits only before its update (so its propagation overlaps the top level).  In the
+// same way a slab top level, which reads its image only in its update, runs its propagation
+// beside the pyramid kernel before it (whose blocks have waited for all earlier work before they
+// let it start).  Not where level L-2 may then start before the pyramid has finished and reads
+// its own pyramid image before it waits (the tile kernel of a level above 0).
+// Measured, us a frame without and with the latter: 640x480, 2 levels, 41.0 and 39.6; 1001x701,
+// 3 levels, 56.0 and 55.6.
 void Filter::chain_pdl(int l, LevelArgs& a) const {
     if (kind_ != Kind::Pyramidal || L_ < 2 || !pdl_chain_) return;
-    auto chained = [&](int m) {
-        const int p = path_of(m, nullptr);
-        return p == kTile || p == kSlab;
-    };
-    if (l == L_ - 1 && chained(L_ - 2)) a.pdl_early_trigger = 1;
+    auto path = [&](int m) { return path_of(m, nullptr); };
+    auto chained = [&](int m) { return path(m) == kTile || path(m) == kSlab; };
+    if (l == L_ - 1) {
+        if (chained(L_ - 2)) a.pdl_early_trigger = 1;
+        if (path(l) == kSlab && (L_ == 2 || path(L_ - 2) != kTile)) a.pdl_late_wait = 1;
+    }
     if (l == L_ - 2 && chained(L_ - 1)) a.pdl_late_wait = 1;
 }
 

@@ -54,7 +54,7 @@ struct LevelArgs {
     int border;
     int first;
     int band;            // rows per warp band (0: chosen from the SM count)
-    // programmatic dependent launch (tile kernel): wait for the preceding kernel only before
+    // programmatic dependent launch (tile and slab kernels): wait for the preceding kernel only before
     // the update (its stages before need nothing that kernel writes), and let the next
     // kernel's blocks start right after this kernel's own wait
     int pdl_late_wait;

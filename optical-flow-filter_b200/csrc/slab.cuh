@@ -406,6 +406,30 @@ __device__ __forceinline__ Q diff_y(const Q& a, const Q& b, const Q& cc, const Q
 
 // ---------------------------------------------------------------- image model and update
 
+// Read-only loads of what the preceding kernel may still be writing when this one starts (the
+// level image, the coarse flow).  Plain __ldg says that the value never changes during the
+// kernel, so the compiler may move it above grid_dep_wait(); volatile keeps their order.
+__device__ __forceinline__ uint32_t ld_waited(const uint32_t* p) {
+    uint32_t v;
+    asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float ld_waited(const float* p) {
+    float v;
+    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float2 ld_waited(const float2* p) {
+    float2 v;
+    asm volatile("ld.global.nc.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float4 ld_waited(const float4* p) {
+    float4 v;
+    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+
 // the lane's four pixels of an image row, clamped at the image edges
 template <typename P>
 struct Image;
@@ -422,7 +446,7 @@ struct Image<uint8_t> {
     }
     // the aligned word holding the columns (rows are 4-byte aligned and padded to words)
     __device__ __forceinline__ Raw raw(int y) const {
-        return __ldg(reinterpret_cast<const uint32_t*>(rowp(p, pitch, min(max(y, 0), H - 1))));
+        return ld_waited(reinterpret_cast<const uint32_t*>(rowp(p, pitch, min(max(y, 0), H - 1))));
     }
     __device__ __forceinline__ Q unit(Raw w) const {
         w = __byte_perm(w, 0, sel);
@@ -447,8 +471,8 @@ struct Image<float> {
     }
     __device__ __forceinline__ Raw raw(int y) const {
         const float* r = rowp(p, pitch, min(max(y, 0), H - 1));
-        if (vec) return __ldg(reinterpret_cast<const float4*>(r));
-        return make_float4(__ldg(r), __ldg(r + o1), __ldg(r + o2), __ldg(r + o3));
+        if (vec) return ld_waited(reinterpret_cast<const float4*>(r));
+        return make_float4(ld_waited(r), ld_waited(r + o1), ld_waited(r + o2), ld_waited(r + o3));
     }
     __device__ __forceinline__ Q unit(const Raw& v) const {
         return Q{make_float2(v.x, v.y), make_float2(v.z, v.w)};
@@ -528,10 +552,10 @@ struct Update {
                 if constexpr (DELTA) {
                     const char* row = rowp(reinterpret_cast<const char*>(a.coarse), (unsigned)a.coarse_pitch, crow);
                     crow = coarse_row(min(y + 1, c.H - 1));
-                    u0 = __ldg(reinterpret_cast<const float2*>(row + cx[0]));
-                    u1 = __ldg(reinterpret_cast<const float2*>(row + cx[1]));
-                    u2 = __ldg(reinterpret_cast<const float2*>(row + cx[2]));
-                    u3 = __ldg(reinterpret_cast<const float2*>(row + cx[3]));
+                    u0 = ld_waited(reinterpret_cast<const float2*>(row + cx[0]));
+                    u1 = ld_waited(reinterpret_cast<const float2*>(row + cx[1]));
+                    u2 = ld_waited(reinterpret_cast<const float2*>(row + cx[2]));
+                    u3 = ld_waited(reinterpret_cast<const float2*>(row + cx[3]));
                 } else {
                     const float* row = rowp(a.io_in, (unsigned)a.io_in_pitch, min(y, c.H - 1));
                     if (a.vec) {
