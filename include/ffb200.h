@@ -296,7 +296,9 @@ ff_status ff_batch_step(ff_batch* batch, const void* frames, void* stream);
 /* Kernel selection (optional; results do not depend on it): the levels that read the
  * previous frame's coarse flow or are top levels (phase A) run the tile-fused kernel below
  * min_pixels pixels (< 0: 200000), every other level the streaming level kernel covers runs
- * it, in bands of band rows (<= 0: the default rule).  Phase-B levels beyond the streaming
+ * it, in bands of band rows (<= 0: the default rule).  With min_pixels < 0, band <= 0 and no
+ * level band set, as at the start, a phase whose levels sum to fewer than 8,000,000 pixels runs
+ * them all by the slab kernel instead.  Phase-B levels beyond the streaming
  * kernel (more than 4 iterations or smoothing passes) add a second tile launch. */
 ff_status ff_batch_set_tuning(ff_batch* batch, long long min_pixels, int band);
 /* Levels of height x width pixels run the streaming kernel in bands of band rows (band <= 0
