@@ -295,7 +295,7 @@ ff_status ff_batch_launches(const ff_batch* batch, int* launches);
 ff_status ff_batch_step(ff_batch* batch, const void* frames, void* stream);
 /* Kernel selection (optional; results do not depend on it): the levels that read the
  * previous frame's coarse flow or are top levels (phase A) run the tile-fused kernel below
- * min_pixels pixels (< 0: 200000), every other level the streaming level kernel covers runs
+ * min_pixels pixels (< 0: the slab kernel below 200000), every other level the streaming level kernel covers runs
  * it, in bands of band rows (<= 0: the default rule).  With min_pixels < 0, band <= 0 and no
  * level band set, as at the start, a phase whose levels sum to fewer than 8,000,000 pixels runs
  * them all by the slab kernel instead.  Phase-B levels beyond the streaming

@@ -411,8 +411,17 @@ bool Batch::streamed(const Filter& f, int l) const {
     const Level& v = f.level(l);
     const int L = f.levels();
     const bool late = L >= 2 && l == L - 2;
-    const long min_px = min_px_ >= 0 ? min_px_ : kDefaultTileBelow;
+    const long min_px = min_px_ >= 0 ? min_px_ : kDefaultBeside;
     return v.item == 1 && (late || (long)v.H * v.W >= min_px) && f.streaming_ok(l);
+}
+
+// Phase-A levels that do not stream run the slab kernel, in the launch beside the streaming one
+// that is the tile kernel's when a pixel limit is set.  Measured on the 64-stream mix: 2008 us a
+// step, 2061 with the tile kernel; levels of less than 1 M pixels there instead of 200,000 gave
+// 2148, those with 3 or more smoothing iterations too 2057.
+bool Batch::slab_beside(const Filter& f, int l) const {
+    const int L = f.levels();
+    return min_px_ < 0 && !(L >= 2 && l == L - 2) && !streamed(f, l) && f.slab_usable(l);
 }
 
 // Levels of phase A (0: tops and levels 0..L-3) or phase B (1: levels L-2).  Below kSlabBelow
@@ -493,16 +502,19 @@ void Batch::set_level_band(int height, int width, int band) {
 }
 
 int Batch::launches_per_step() const {
-    bool stream_a = false, stream_b = false, tile_a = false, tile_b = false;
+    bool stream_a = false, stream_b = false, tile_a = false, tile_b = false, slab_a = false;
+    const bool mixed_a = !slab_phase(0);
     for (auto& f : f_) {
         const int L = f->levels();
         for (int l = 0; l < L; ++l) {
             const bool late = L >= 2 && l == L - 2;
-            (streamed(*f, l) ? (late ? stream_b : stream_a) : (late ? tile_b : tile_a)) = true;
+            if (mixed_a && slab_beside(*f, l)) slab_a = true;
+            else (streamed(*f, l) ? (late ? stream_b : stream_a) : (late ? tile_b : tile_a)) = true;
         }
     }
     // the ingest and pyramid launch, one per pyramid depth beyond 2, one per phase and kernel
-    return 1 + std::max(max_levels_ - 3, 0) + (int)stream_a + (int)stream_b + (int)tile_a + (int)tile_b;
+    return 1 + std::max(max_levels_ - 3, 0) + (int)stream_a + (int)stream_b + (int)tile_a + (int)tile_b +
+           (int)slab_a;
 }
 
 bool Batch::matches(const Table& t) const {
@@ -580,21 +592,27 @@ void Batch::build(Table& t) {
     }
     // phase A: top levels and levels 0..L-3 (they read the previous frame's coarse flow);
     // phase B: levels L-2 (they read this frame's top-level flow).  Streamed levels go to the
-    // phase's streaming launch, the others to its tile launch.
+    // phase's streaming launch, the others to the slab or tile launch beside it.
     std::vector<StreamJob> sj[2];
     std::vector<TileJob> tj[2];
-    // slab phases: the levels that would stream in sl[ph][0], the others in sl[ph][1]
+    // slab phases: the levels that would stream in sl[ph][0], the others in sl[ph][1]; phase A
+    // otherwise: the levels of slab_beside in sl[0][1]
     std::vector<SlabJob> sl[2][2];
     int slblocks[2][2] = {};
     size_t slsmem[2][2] = {};
+    const bool all_slab[2] = {slab_phase(0), slab_phase(1)};
     for (int ph = 0; ph < 2; ++ph) {
-        if (!slab_phase(ph)) continue;
         SlabPlan plan;
         for (auto& f : f_) {
             const int L = f->levels();
             for (int l = 0; l < L; ++l) {
                 if ((L >= 2 && l == L - 2) != (ph == 1)) continue;
+                if (!all_slab[ph] && !slab_beside(*f, l)) continue;
                 const Level& v = f->level(l);
+                // a batch is accepted or refused whatever its tuning: what does not stream has
+                // to fit the tile kernel, which setting a pixel limit would run
+                size_t tile_smem = 0;
+                if (!streamed(*f, l)) batch_geom(v.delta, v.iters, v.smooth, v.W, v.H, &tile_smem);
                 plan.items.push_back({f.get(), l, streamed(*f, l) ? 0 : 1,
                                       (v.delta ? 185.0 : 80.0) * v.iters + 330.0 + 110.0 * v.smooth});
             }
@@ -625,7 +643,7 @@ void Batch::build(Table& t) {
         for (int l = 0; l < L; ++l) {
             const Level& v = f->level(l);
             const int ph = L >= 2 && l == L - 2 ? 1 : 0;
-            if (!sl[ph][0].empty() || !sl[ph][1].empty()) continue;
+            if (all_slab[ph] || slab_beside(*f, l)) continue;
             if (streamed(*f, l)) {
                 StreamJob j{};
                 j.a = f->level_args(l);
@@ -689,8 +707,8 @@ void Batch::build(Table& t) {
         t.gen.push_back(f->config_generation());
     }
     t.tune_gen = tune_gen_;
-    // capture: the deeper pyramid depths; phase A's streaming launch, with its tile launch on
-    // a branch beside it (the small levels fill the streaming launch's tail); phase B's
+    // capture: the deeper pyramid depths; phase A's streaming launch, with its slab or tile
+    // launch on a branch beside it (the small levels fill the streaming launch's tail); phase B's
     // launches after both
     cudaGraph_t g = nullptr;
     check_cuda(cudaStreamBeginCapture(cap_, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
@@ -706,7 +724,8 @@ void Batch::build(Table& t) {
             ++launches;
         }
     for (int ph = 0; ph < 2; ++ph) {
-        const bool branch = (ph == 0 && !tj[0].empty() && !sj[0].empty()) || (!sl[ph][0].empty() && !sl[ph][1].empty());
+        const bool branch = (ph == 0 && !tj[0].empty() && !sj[0].empty()) ||
+                            ((!sl[ph][0].empty() || !sj[ph].empty()) && !sl[ph][1].empty());
         if (branch) {
             ok(cudaEventRecord(fork_, cap_));
             ok(cudaStreamWaitEvent(side_, fork_, 0));

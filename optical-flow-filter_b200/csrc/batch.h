@@ -8,14 +8,16 @@
 //               its level-0 image and builds pyramid levels 1 and 2 from it
 //   (deeper pyramid levels, when a stream has more than 3: one launch per depth)
 //   levels A    one streaming-kernel launch over every top level and every delta level that
-//               reads the previous frame's coarse flow (levels 0..L-3)
+//               reads the previous frame's coarse flow (levels 0..L-3), with a slab-kernel
+//               launch over the small ones beside it
 //   levels B    one streaming-kernel launch over the levels L-2, which read this frame's
 //               unsmoothed top-level flow
 //
 // A phase launch walks a device table of jobs (one per stream-level), each job a contiguous
 // range of blocks running the instantiation of the streaming kernel for its (delta,
 // iterations, smoothing) (level_mega.cu).  Levels the streaming kernel does not cover (more
-// than 4 iterations or smoothing passes) go to one tile-kernel launch per phase.  The phase
+// than 4 iterations or smoothing passes) go to the slab launch in phase A and to a tile-kernel
+// launch in phase B.  Small batches run both phases by the slab kernel.  The phase
 // launches of a step are replayed from a CUDA graph.  Every stream's results are those of the
 // same stream filtered alone, whatever the tuning.
 #pragma once
@@ -51,11 +53,11 @@ public:
     int launches_per_step() const;
     // advance every stream by one frame read from `frames` (frame_bytes() bytes on the device)
     void step(const void* frames, cudaStream_t s);
-    // phase-A levels of fewer than min_pixels pixels (< 0: kDefaultTileBelow) run the tile
-    // kernel, every other level the streaming kernel covers runs it, in bands of `band` rows
-    // (<= 0: chosen per step)
+    // phase-A levels of fewer than min_pixels pixels run the tile kernel (< 0: of fewer than
+    // kDefaultBeside the slab kernel), every other level the streaming kernel covers runs it, in
+    // bands of `band` rows (<= 0: chosen per step)
     void set_tuning(long min_pixels, int band);
-    static constexpr long kDefaultTileBelow = 200000;
+    static constexpr long kDefaultBeside = 200000;
     // A phase of less than kSlabBelow pixels runs its levels by the slab kernel, in the launches
     // that otherwise are its streaming and its tile launch, unless set_tuning or set_level_band
     // ask for something else
@@ -71,6 +73,7 @@ private:
     void release_table(Table& t);
     bool streamed(const Filter& f, int l) const;
     bool slab_phase(int phase) const;
+    bool slab_beside(const Filter& f, int l) const;
     int band_of(const Level& v, int rule_band) const;
 
     std::vector<std::unique_ptr<Filter>> f_;

@@ -619,8 +619,8 @@ class BatchFlowFilter:
 
     def setTuning(self, minPixels: int = -1, band: int = 0) -> None:
         """Top levels and levels reading the previous frame's coarse flow (phase A) below
-        ``minPixels`` pixels run the tile kernel (-1: 200000), every other level the streaming
-        kernel covers runs it in bands of ``band`` rows (0: the default rule).  With the
+        ``minPixels`` pixels run the tile kernel (-1: below 200000 the slab kernel), every
+        other level the streaming kernel covers runs it in bands of ``band`` rows (0: the default rule).  With the
         defaults and no level band, a phase of fewer than 8,000,000 pixels runs all its
         levels by the slab kernel.  Results are unchanged."""
         call("ff_batch_set_tuning", self._h, int(minPixels), int(band))
