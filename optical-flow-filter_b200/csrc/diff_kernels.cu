@@ -2103,7 +2103,10 @@ struct Driver {
         auto slab = [&](int l) { return std::is_same<T, float>::value && slab_available(l < top, g.N[l], g.S[l]); };
         // top level: flow propagation, update, smoothing
         if (slab(top)) {
-            T* fu = compact && fu_out ? fu_out : tp + tape.sm[top][0];
+            // the unsmoothed flow: level L-2 reads it from the tape, and the adjoint; a single level
+            // without a tape has no reader but the caller (whose buffer may be at any element)
+            const bool direct = compact && L == 1 && fu_out && (uintptr_t)fu_out % (2 * sizeof(T)) == 0;
+            T* fu = direct ? fu_out : tp + tape.sm[top][0];
             if constexpr (std::is_same<T, float>::value)
                 level_slab(top, first, img(top), gamma, weights, in, out, nullptr, fu, top == 0 ? y_out : nullptr,
                            compact ? nullptr : &tape, tp);
