@@ -49,8 +49,10 @@ cudaError_t device_malloc_pitch(void** p, size_t* pitch, size_t width_bytes, siz
 }
 
 // Rows are allocated with room for one extra pixel (and a 4-byte multiple), so the fused
-// kernels' aligned pair copies of columns (W-1, W) stay inside the allocation.
-void Buf::alloc(int h_, int w_, int bpp_) {
+// kernels' aligned pair copies of columns (W-1, W) stay inside the allocation.  The clearing
+// runs on the stream that uses the buffer: the filters' streams are not ordered after the
+// default stream, where it could still be on its way while a kernel already writes the buffer.
+void Buf::alloc(int h_, int w_, int bpp_, cudaStream_t s) {
     release();
     h = h_;
     w = w_;
@@ -58,7 +60,7 @@ void Buf::alloc(int h_, int w_, int bpp_) {
     if (h <= 0 || w <= 0) return;
     const size_t row = ((size_t)(w + 1) * bpp + 3) & ~(size_t)3;
     check_cuda(device_malloc_pitch(&p, &pitch, row, (size_t)h), "cudaMallocPitch");
-    check_cuda(cudaMemset2D(p, pitch, 0, row, (size_t)h), "cudaMemset2D");
+    check_cuda(cudaMemset2DAsync(p, pitch, 0, row, (size_t)h, s), "cudaMemset2DAsync");
 }
 
 void Buf::release() {
@@ -71,13 +73,13 @@ void Buf::clear(cudaStream_t s) {
     if (p) check_cuda(cudaMemset2DAsync(p, pitch, 0, row_bytes(), (size_t)h, s), "cudaMemset2DAsync");
 }
 
-void Level::alloc_state() {
+void Level::alloc_state(cudaStream_t s) {
     for (int k = 0; k < 2; ++k) {
-        fs[k].alloc(H, W, 8);
-        io[k].alloc(H, W, 4);
-        if (delta) d[k].alloc(H, W, 8);
+        fs[k].alloc(H, W, 8, s);
+        io[k].alloc(H, W, 4, s);
+        if (delta) d[k].alloc(H, W, 8, s);
     }
-    if (!delta) fu.alloc(H, W, 8);
+    if (!delta) fu.alloc(H, W, 8, s);
 }
 
 // Same index as the device's upmap_index (common.cuh): u = x/(W-1) rounded to float,
@@ -93,26 +95,27 @@ static int upmap_index_host(int x, int W, int Wc) {
     return (int)i;
 }
 
-void Level::build_coarse_rows() {
+void Level::build_coarse_rows(cudaStream_t s) {
     if (!delta || Hc <= 0) return;
     std::vector<int> t(H);
     for (int y = 0; y < H; ++y) t[y] = upmap_index_host(y, H, Hc);
-    coarse_rows.alloc(1, H, 4);
-    check_cuda(cudaMemcpy(coarse_rows.p, t.data(), t.size() * sizeof(int), cudaMemcpyHostToDevice), "coarse rows");
+    coarse_rows.alloc(1, H, 4, s);
+    check_cuda(cudaMemcpyAsync(coarse_rows.p, t.data(), t.size() * sizeof(int), cudaMemcpyHostToDevice, s), "coarse rows");
+    check_cuda(cudaStreamSynchronize(s), "coarse rows");  // in place before work on any stream
 }
 
-void Level::alloc_scratch() {
+void Level::alloc_scratch(cudaStream_t s) {
     if (a0.p) return;
-    a0.alloc(H, W, 4);
-    grad.alloc(H, W, 8);
-    fp.alloc(H, W, 8);
-    t1.alloc(H, W, 8);
+    a0.alloc(H, W, 4, s);
+    grad.alloc(H, W, 8, s);
+    fp.alloc(H, W, 8, s);
+    t1.alloc(H, W, 8, s);
     if (delta) {
-        ip.alloc(H, W, 4);
-        dp.alloc(H, W, 8);
-        t2.alloc(H, W, 4);
-        t3.alloc(H, W, 8);
-        fut.alloc(H, W, 8);
+        ip.alloc(H, W, 4, s);
+        dp.alloc(H, W, 8, s);
+        t2.alloc(H, W, 4, s);
+        t3.alloc(H, W, 8, s);
+        fut.alloc(H, W, 8, s);
     }
 }
 
@@ -150,7 +153,7 @@ Filter::Filter(Kind kind, int H, int W, int levels, int item, bool own_input)
         lv_.resize(L_);
         if (kind == Kind::Pyramidal) {
             // ImagePyramid::configure: integer halving, X then Y (pyramid.cu:74-83)
-            input_.alloc(H, W, item);
+            input_.alloc(H, W, item, stream_);
             int h = H, w = W;
             pyr_.resize(L_ - 1);
             for (int l = 0; l < L_; ++l) {
@@ -159,7 +162,7 @@ Filter::Filter(Kind kind, int H, int W, int levels, int item, bool own_input)
                     h /= 2;
                     if (h <= 0 || w <= 0)
                         throw Error(FF_ERR_INVALID_ARGUMENT, "pyramid level " + std::to_string(l) + " has zero size");
-                    pyr_[l - 1].alloc(h, w, item);
+                    pyr_[l - 1].alloc(h, w, item, stream_);
                 }
                 Level& v = lv_[l];
                 v.delta = l < L_ - 1;
@@ -173,7 +176,7 @@ Filter::Filter(Kind kind, int H, int W, int levels, int item, bool own_input)
             for (int l = 0; l < L_ - 1; ++l) {
                 lv_[l].Hc = lv_[l + 1].H;
                 lv_[l].Wc = lv_[l + 1].W;
-                lv_[l].build_coarse_rows();
+                lv_[l].build_coarse_rows(stream_);
             }
         } else {
             Level& v = lv_[0];
@@ -182,7 +185,7 @@ Filter::Filter(Kind kind, int H, int W, int levels, int item, bool own_input)
             v.W = W;
             v.item = item;
             if (own_input) {
-                input_.alloc(H, W, item);
+                input_.alloc(H, W, item, stream_);
                 v.img = input_.p;
                 v.img_pitch = input_.pitch;
                 v.img_owned = true;
@@ -190,7 +193,7 @@ Filter::Filter(Kind kind, int H, int W, int levels, int item, bool own_input)
         }
         // configure() defaults: FlowUpdate/DeltaFlowUpdate(gamma 1, maxflow 1),
         // FlowSmoother(1), FlowPropagator(1), border 3 (flowfilter.cu:100-107, 393-402)
-        for (Level& v : lv_) v.alloc_state();
+        for (Level& v : lv_) v.alloc_state(stream_);
         check_cuda(cudaDeviceSynchronize(), "configure");
     } catch (...) {
         for (Level& v : lv_) v.release();
@@ -244,7 +247,7 @@ void Filter::process_host_async(const ff_image& in, ff_image& out, cudaStream_t 
         check_cuda(cudaStreamCreateWithFlags(&p->in, cudaStreamNonBlocking), "cudaStreamCreate");
         check_cuda(cudaStreamCreateWithFlags(&p->out, cudaStreamNonBlocking), "cudaStreamCreate");
         for (int k = 0; k < 2; ++k) {
-            p->staging[k].alloc(H_, W_, item_);
+            p->staging[k].alloc(H_, W_, item_, p->in);
             for (cudaEvent_t* e : {&p->h2d[k], &p->computed[k], &p->d2h[k]}) {
                 check_cuda(cudaEventCreateWithFlags(e, cudaEventDisableTiming), "cudaEventCreate");
                 check_cuda(cudaEventRecord(*e, stream_), "cudaEventRecord");
@@ -483,7 +486,7 @@ void Filter::set_external_coarse(const void* flow, size_t pitch, int Hc, int Wc)
     v.coarse_pitch = pitch;
     v.Hc = Hc;
     v.Wc = Wc;
-    v.build_coarse_rows();
+    v.build_coarse_rows(stream_);
 }
 
 void Filter::coarse_of(int l, const void** p, size_t* pitch, int* Hc, int* Wc) const {
@@ -505,7 +508,7 @@ void Filter::coarse_of(int l, const void** p, size_t* pitch, int* Hc, int* Wc) c
 // ------------------------------------------------------------------ unfused path
 void Filter::model_unfused(int l, cudaStream_t s) {
     Level& v = lv_[l];
-    v.alloc_scratch();
+    v.alloc_scratch(s);
     check_cuda(launch_image_model(v.img, v.img_pitch, v.item, v.H, v.W, (float*)v.a0.p, v.a0.pitch,
                                   (float*)v.grad.p, v.grad.pitch, s),
                "image model");
@@ -513,7 +516,7 @@ void Filter::model_unfused(int l, cudaStream_t s) {
 
 void Filter::propagate_unfused(int l, cudaStream_t s) {
     Level& v = lv_[l];
-    v.alloc_scratch();
+    v.alloc_scratch(s);
     const Buf& fs = v.fs[cur_];
     if (!v.delta) {
         check_cuda(launch_propagate((const float*)fs.p, fs.pitch, v.H, v.W, v.iters, v.border, (float*)v.fp.p,
@@ -533,7 +536,7 @@ void Filter::propagate_unfused(int l, cudaStream_t s) {
 
 void Filter::update_unfused(int l, cudaStream_t s) {
     Level& v = lv_[l];
-    v.alloc_scratch();
+    v.alloc_scratch(s);
     const int nxt = cur_ ^ 1;
     if (!v.delta) {
         const Buf& io = v.io[cur_];
@@ -778,7 +781,7 @@ void Filter::autotune(int reps, void* flush, size_t flush_bytes) {
     Buf keep;
     Level& top = lv_[L_ - 1];
     if (!top.delta && top.fu.p) {
-        keep.alloc(top.fu.h, top.fu.w, top.fu.bpp);
+        keep.alloc(top.fu.h, top.fu.w, top.fu.bpp, stream_);
         check_cuda(cudaMemcpy2DAsync(keep.p, keep.pitch, top.fu.p, top.fu.pitch, top.fu.row_bytes(), top.fu.h,
                                      cudaMemcpyDeviceToDevice, stream_), "autotune");
     }
@@ -821,7 +824,7 @@ void Filter::autotune(int reps, void* flush, size_t flush_bytes) {
     std::vector<std::vector<Choice>> timed(L_);
     for (int l = L_ - 1; l >= 0; --l) {
         Level& v = lv_[l];
-        v.alloc_scratch();  // allocations cannot happen inside a capture
+        v.alloc_scratch(stream_);  // allocations cannot happen inside a capture
         std::vector<Choice>& c = timed[l];
         c.push_back({time_it([&](cudaStream_t st) { step_level_unfused(l, st); }), kPerStage, 0});
         if (fused_ok(l)) {
@@ -959,11 +962,11 @@ float Filter::time_level(int l, int reps, void* flush, size_t flush_bytes) {
     Level& top = lv_[L_ - 1];
     Buf keep;
     if (!top.delta && top.fu.p) {  // getFlow() result / coarse input: restored afterwards
-        keep.alloc(top.fu.h, top.fu.w, top.fu.bpp);
+        keep.alloc(top.fu.h, top.fu.w, top.fu.bpp, stream_);
         check_cuda(cudaMemcpy2DAsync(keep.p, keep.pitch, top.fu.p, top.fu.pitch, top.fu.row_bytes(), top.fu.h,
                                      cudaMemcpyDeviceToDevice, stream_), "time_level");
     }
-    if (path_of(l, nullptr) == kPerStage) lv_[l].alloc_scratch();
+    if (path_of(l, nullptr) == kPerStage) lv_[l].alloc_scratch(stream_);
     cudaGraph_t g = nullptr;
     cudaGraphExec_t ge = nullptr;
     check_cuda(cudaStreamBeginCapture(cap_, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
@@ -1100,7 +1103,7 @@ void Filter::compute_async(cudaStream_t s) {
         if (!ge) {
             // per-stage levels need their scratch before the capture (no allocation inside it)
             for (int l = 0; l < L_; ++l)
-                if (path_of(l, nullptr) == kPerStage) lv_[l].alloc_scratch();
+                if (path_of(l, nullptr) == kPerStage) lv_[l].alloc_scratch(s);
             // capture this parity's frame once; the buffers it names alternate per frame
             check_cuda(cudaStreamBeginCapture(cap_, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
             try {

@@ -47,7 +47,8 @@ struct Buf {
     size_t pitch = 0;
     int h = 0, w = 0;   // pixels
     int bpp = 0;        // bytes per pixel
-    void alloc(int h_, int w_, int bpp_);
+    // zeroed by stream s: its later work, and what waits for it, finds the buffer cleared
+    void alloc(int h_, int w_, int bpp_, cudaStream_t s);
     void release();
     void clear(cudaStream_t s);
     size_t row_bytes() const { return (size_t)w * bpp; }
@@ -80,11 +81,11 @@ struct Level {
     int tuned_path = -1;         // autotuned: -1 not tuned, else a Path
     int tuned_band = 0;          // streaming, slab kernel: band, slab rows; tile kernel: tile shape (0 automatic)
     Buf coarse_rows;             // int per row: coarse row its update reads (delta levels)
-    void build_coarse_rows();
+    void build_coarse_rows(cudaStream_t s);
     // scratch of the unfused path (allocated on first use)
     Buf a0, grad, fp, ip, dp, t1, t2, t3, fut;
-    void alloc_state();
-    void alloc_scratch();
+    void alloc_state(cudaStream_t s);
+    void alloc_scratch(cudaStream_t s);
     void release();
 };
 
