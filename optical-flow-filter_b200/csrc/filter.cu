@@ -104,18 +104,24 @@ void Level::build_coarse_rows(cudaStream_t s) {
     check_cuda(cudaStreamSynchronize(s), "coarse rows");  // in place before work on any stream
 }
 
+// all of it or, if an allocation fails, none
 void Level::alloc_scratch(cudaStream_t s) {
     if (a0.p) return;
-    a0.alloc(H, W, 4, s);
-    grad.alloc(H, W, 8, s);
-    fp.alloc(H, W, 8, s);
-    t1.alloc(H, W, 8, s);
-    if (delta) {
-        ip.alloc(H, W, 4, s);
-        dp.alloc(H, W, 8, s);
-        t2.alloc(H, W, 4, s);
-        t3.alloc(H, W, 8, s);
-        fut.alloc(H, W, 8, s);
+    try {
+        a0.alloc(H, W, 4, s);
+        grad.alloc(H, W, 8, s);
+        fp.alloc(H, W, 8, s);
+        t1.alloc(H, W, 8, s);
+        if (delta) {
+            ip.alloc(H, W, 4, s);
+            dp.alloc(H, W, 8, s);
+            t2.alloc(H, W, 4, s);
+            t3.alloc(H, W, 8, s);
+            fut.alloc(H, W, 8, s);
+        }
+    } catch (...) {
+        for (Buf* b : {&a0, &grad, &fp, &ip, &dp, &t1, &t2, &t3, &fut}) b->release();
+        throw;
     }
 }
 
@@ -1098,12 +1104,13 @@ void Filter::compute_async(cudaStream_t s) {
     begin_on(s);
     bool any_first = false;
     for (const Level& v : lv_) any_first |= v.first;
+    // per-stage levels get their scratch before anything is queued: a failure leaves no part of
+    // a frame behind, and there is no allocation inside a capture
+    for (int l = 0; l < L_; ++l)
+        if (!lv_[l].a0.p && path_of(l, nullptr) == kPerStage) lv_[l].alloc_scratch(s);
     if (graphs_ && !any_first && prof_count_ >= prof_cap_) {
         cudaGraphExec_t& ge = graph_exec_[cur_];
         if (!ge) {
-            // per-stage levels need their scratch before the capture (no allocation inside it)
-            for (int l = 0; l < L_; ++l)
-                if (path_of(l, nullptr) == kPerStage) lv_[l].alloc_scratch(s);
             // capture this parity's frame once; the buffers it names alternate per frame
             check_cuda(cudaStreamBeginCapture(cap_, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
             try {
