@@ -406,30 +406,6 @@ __device__ __forceinline__ Q diff_y(const Q& a, const Q& b, const Q& cc, const Q
 
 // ---------------------------------------------------------------- image model and update
 
-// Read-only loads of what the preceding kernel may still be writing when this one starts (the
-// level image, the coarse flow).  Plain __ldg says that the value never changes during the
-// kernel, so the compiler may move it above grid_dep_wait(); volatile keeps their order.
-__device__ __forceinline__ uint32_t ld_waited(const uint32_t* p) {
-    uint32_t v;
-    asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ float ld_waited(const float* p) {
-    float v;
-    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ float2 ld_waited(const float2* p) {
-    float2 v;
-    asm volatile("ld.global.nc.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ float4 ld_waited(const float4* p) {
-    float4 v;
-    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
-    return v;
-}
-
 // the lane's four pixels of an image row, clamped at the image edges
 template <typename P>
 struct Image;
@@ -515,7 +491,7 @@ struct Update {
         c.run_of(r2, y0, y1);
         if (y0 < y1) {
             const Image<P> img(a, c);
-            const float gamma = a.gamma_dev ? __ldg(a.gamma_dev) : a.gamma;
+            const float gamma = a.gamma_dev ? ld_waited(a.gamma_dev) : a.gamma;
             const float2 g = make_float2(gamma, gamma);
             const float m = a.maxflow, hm = __fmul_rn(0.5f, m);
             const bool first = a.first != 0, vec = c.vec;
@@ -559,11 +535,11 @@ struct Update {
                 } else {
                     const float* row = rowp(a.io_in, (unsigned)a.io_in_pitch, min(y, c.H - 1));
                     if (a.vec) {
-                        const float4 v = __ldg(reinterpret_cast<const float4*>(row + c.wcol));
+                        const float4 v = ld_waited(reinterpret_cast<const float4*>(row + c.wcol));
                         old_top = Q{make_float2(v.x, v.y), make_float2(v.z, v.w)};
                     } else {
-                        old_top = Q{make_float2(__ldg(row + cc[0]), __ldg(row + cc[1])),
-                                    make_float2(__ldg(row + cc[2]), __ldg(row + cc[3]))};
+                        old_top = Q{make_float2(ld_waited(row + cc[0]), ld_waited(row + cc[1])),
+                                    make_float2(ld_waited(row + cc[2]), ld_waited(row + cc[3]))};
                     }
                 }
             };
@@ -622,7 +598,7 @@ struct Update {
                     if (!DELTA && a.d_out) {  // a state field that top levels pass on unchanged
                         const float2* d = rowp(reinterpret_cast<const float2*>(a.d_in), (unsigned)a.d_in_pitch, y) + c.c0;
                         float2* o = rowp(reinterpret_cast<float2*>(a.d_out), (unsigned)a.d_out_pitch, y) + c.c0;
-                        for (int j = 0; j < nout; ++j) o[j] = __ldg(d + j);
+                        for (int j = 0; j < nout; ++j) o[j] = ld_waited(d + j);
                     }
                 }
             }
@@ -766,6 +742,8 @@ __device__ __forceinline__ void make_ctx(const LevelArgs& a, const Geom& g, int 
 }
 
 // the previous frame's state of the slab's rows into the planes, all rows in flight at once
+// (the filters' own rows are always aligned, so a load that runs before grid_dep_wait() comes from
+// L2, where the writes of completed kernels are)
 template <bool DELTA>
 __device__ __forceinline__ void load_state(const LevelArgs& a, const Ctx& c, int sy1) {
     constexpr int ROWB = planes(DELTA) * kPlane;
@@ -847,7 +825,7 @@ template <bool DELTA, bool TAPE>
 __device__ __forceinline__ void smooth(const Ctx& c, const LevelArgs& a, int S, const Tape& tape) {
     typename Smooth<DELTA>::W5 w;
 #pragma unroll
-    for (int j = 0; j < 5; ++j) w.k[j] = a.weights ? __ldg(a.weights + j) : kBox;
+    for (int j = 0; j < 5; ++j) w.k[j] = a.weights ? ld_waited(a.weights + j) : kBox;
 #pragma unroll 1
     for (int s = 1; s <= S; ++s) {
         const int r = 2 * (S - s);

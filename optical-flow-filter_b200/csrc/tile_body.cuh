@@ -173,7 +173,8 @@ __device__ __forceinline__ void tile_body(const LevelArgs& a, const Geom& g, int
     // pdl_late_wait (a delta level launched right after its top level) the state load,
     // propagation and image model read only the previous frame's state and an image that
     // was complete before the preceding kernel passed its own wait, so the wait moves to
-    // just before the update, the first stage that reads the coarse flow.
+    // just before the update, the first stage that reads the coarse flow.  What is read before
+    // the wait comes from L2 (__ldcg), where the writes of completed kernels are.
     const bool late_wait = a.pdl_late_wait != 0;
     if (!late_wait) grid_dep_wait();
     if (a.pdl_early_trigger) grid_dep_launch();
@@ -185,13 +186,13 @@ __device__ __forceinline__ void tile_body(const LevelArgs& a, const Geom& g, int
     const int SW = g.SW, NS = g.SW * g.SH;
     const int B = a.border;
     // kernel parameters used per pixel, held in registers
-    const float2* __restrict__ fs_in = reinterpret_cast<const float2*>(a.fs_in);
-    const float2* __restrict__ d_in = reinterpret_cast<const float2*>(a.d_in);
-    const float* __restrict__ io_in = a.io_in;
+    const float2* fs_in = reinterpret_cast<const float2*>(a.fs_in);
+    const float2* d_in = reinterpret_cast<const float2*>(a.d_in);
+    const float* io_in = a.io_in;
     const size_t fs_in_p = a.fs_in_pitch, d_in_p = a.d_in_pitch, io_in_p = a.io_in_pitch;
-    const P* __restrict__ img_in = reinterpret_cast<const P*>(a.img);
+    const P* img_in = reinterpret_cast<const P*>(a.img);
     const size_t img_p = a.img_pitch;
-    const float2* __restrict__ coarse = reinterpret_cast<const float2*>(a.coarse);
+    const float2* coarse = reinterpret_cast<const float2*>(a.coarse);
     const size_t coarse_p = a.coarse_pitch;
     const int* __restrict__ coarse_rows = a.coarse_rows;
     float* const d_out = a.d_out;
@@ -228,10 +229,10 @@ __device__ __forceinline__ void tile_body(const LevelArgs& a, const Geom& g, int
             xa(g.R), xb(g.R), ya(g.R), yb(g.R), SW, sidx(xa(g.R), ya(g.R)),
             [&](int x, int y, int) {
                 In v;
-                v.f = __ldg(grow<float2>(fs_in, fs_in_p, y) + x);
+                v.f = __ldcg(grow<float2>(fs_in, fs_in_p, y) + x);
                 if constexpr (DELTA) {
-                    v.d = __ldg(grow<float2>(d_in, d_in_p, y) + x);
-                    v.i = __ldg(grow<float>(io_in, io_in_p, y) + x);
+                    v.d = __ldcg(grow<float2>(d_in, d_in_p, y) + x);
+                    v.i = __ldcg(grow<float>(io_in, io_in_p, y) + x);
                 }
                 return v;
             },
@@ -346,7 +347,7 @@ __device__ __forceinline__ void tile_body(const LevelArgs& a, const Geom& g, int
     } else {
         walk(
             xa(rI), xb(rI), ya(rI), yb(rI), IW, iidx(xa(rI), ya(rI)),
-            [&](int x, int y, int) { return __ldg(grow<P>(img_in, img_p, y) + x); },
+            [&](int x, int y, int) { return __ldcg(grow<P>(img_in, img_p, y) + x); },
             [&](int, int, int k, P v) { img[k] = Pix<P>::get(v); });
     }
     if constexpr (DELTA) {
@@ -419,9 +420,9 @@ __device__ __forceinline__ void tile_body(const LevelArgs& a, const Geom& g, int
                     u.old = is[k];
                     u.f = ds[k];
                     const int cr = __ldg(coarse_rows + y);
-                    u.up = __ldg(grow<float2>(coarse, coarse_p, cr) + ccol[x - x0 + S2]);
+                    u.up = grow<float2>(coarse, coarse_p, cr)[ccol[x - x0 + S2]];
                 } else {
-                    u.old = __ldg(grow<float>(io_in, io_in_p, y) + x);
+                    u.old = grow<float>(io_in, io_in_p, y)[x];
                     u.f = fs[k];
                 }
                 return u;
