@@ -79,7 +79,7 @@ constexpr int P2X = 64, P2Y = 16;  // level-1 tile of the ingest launch (blocks 
 // each direction, the columns from a 4-byte boundary (4 before)
 constexpr int S0Y = 2 * P2Y + 5, S0X = 2 * P2X + 8;
 // block_job[b]: the job of block b (a table, so a block finds its job in one load)
-__global__ void __launch_bounds__(256, 6) ingest_pyr_k(const uint8_t* __restrict__ frames,
+__global__ void __launch_bounds__(256, 6) ingest_pyr_k(const uint8_t* frames,
                                                        const IngestJob* __restrict__ jobs,
                                                        const unsigned short* __restrict__ block_job) {
     __shared__ __align__(16) uint8_t s0[S0Y][S0X];
@@ -98,19 +98,24 @@ __global__ void __launch_bounds__(256, 6) ingest_pyr_k(const uint8_t* __restrict
         const int xe = tx == j.tiles_x - 1 ? W : min(x0 + 2 * P2X, W);
         const int ye = ty == j.tiles_y - 1 ? H : min(y0 + 2 * P2Y, H);
         const int wv = xe - x0, rows = ye - y0;
-        if (words) {
-            const int wq = wv >> 2;
-            for (int k = tid; k < rows * wq; k += 256) {
-                const int r = k / wq, c = k - r * wq;
-                reinterpret_cast<uint32_t*>(j.dst + (size_t)(y0 + r) * j.dst_pitch + x0)[c] =
-                    __ldg(reinterpret_cast<const uint32_t*>(src + (size_t)(y0 + r) * W + x0) + c);
-            }
-        } else {
-            for (int k = tid; k < rows * wv; k += 256) {
-                const int r = k / wv, c = k - r * wv;
-                j.dst[(size_t)(y0 + r) * j.dst_pitch + x0 + c] = __ldg(src + (size_t)(y0 + r) * W + x0 + c);
-            }
-        }
+        // a warp per row, four rows in flight per lane before their stores
+        auto copy = [&](auto px, int columns) {
+            using V = decltype(px);
+            for (int c = tid & 31; c < columns; c += 32)
+                for (int r = tid >> 5; r < rows; r += 32) {
+                    V v[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (r + 8 * u < rows)
+                            v[u] = reinterpret_cast<const V*>(src + (size_t)(y0 + r + 8 * u) * W + x0)[c];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (r + 8 * u < rows)
+                            reinterpret_cast<V*>(j.dst + (size_t)(y0 + r + 8 * u) * j.dst_pitch + x0)[c] = v[u];
+                }
+        };
+        if (words) copy(uint32_t{}, wv >> 2);
+        else copy(uint8_t{}, wv);
         return;
     }
     const int x1 = tx * P2X, y1 = ty * P2Y;
@@ -125,11 +130,11 @@ __global__ void __launch_bounds__(256, 6) ingest_pyr_k(const uint8_t* __restrict
                 const uint8_t* row = src + (size_t)min(max(Y0 + r, 0), H - 1) * W;
                 const int x = X0 + 4 * c;
                 if (x >= 0 && x + 3 < W) {
-                    v[u] = __ldg(reinterpret_cast<const uint32_t*>(row + x));
+                    v[u] = *reinterpret_cast<const uint32_t*>(row + x);
                 } else {  // a word beyond an edge: its clamped bytes
                     uint32_t w = 0;
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) w |= (uint32_t)__ldg(row + min(max(x + q, 0), W - 1)) << (8 * q);
+                    for (int q = 0; q < 4; ++q) w |= (uint32_t)row[min(max(x + q, 0), W - 1)] << (8 * q);
                     v[u] = w;
                 }
             }
@@ -145,7 +150,7 @@ __global__ void __launch_bounds__(256, 6) ingest_pyr_k(const uint8_t* __restrict
 #pragma unroll
         for (int u = 0; u < NS; ++u) {
             const int e = tid + 256 * u, r = e / S0X, c = e - r * S0X;
-            if (e < S0Y * S0X) v[u] = __ldg(src + (size_t)min(max(Y0 + r, 0), H - 1) * W + min(max(X0 + c, 0), W - 1));
+            if (e < S0Y * S0X) v[u] = src[(size_t)min(max(Y0 + r, 0), H - 1) * W + min(max(X0 + c, 0), W - 1)];
         }
 #pragma unroll
         for (int u = 0; u < NS; ++u) {

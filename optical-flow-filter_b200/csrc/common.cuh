@@ -32,11 +32,12 @@ struct CView {
         return reinterpret_cast<const T*>(reinterpret_cast<const char*>(ptr) + (size_t)y * pitch);
     }
     __host__ __device__ __forceinline__ const T& at(int x, int y) const { return row(y)[x]; }
-    // clamp-to-edge read: the reference's textures use cudaAddressModeClamp
+    // clamp-to-edge read: the reference's textures use cudaAddressModeClamp (a plain load: see
+    // ld_waited, launch.cuh)
     __device__ __forceinline__ T clamped(int x, int y) const {
         x = min(max(x, 0), w - 1);
         y = min(max(y, 0), h - 1);
-        return __ldg(row(y) + x);
+        return row(y)[x];
     }
 };
 

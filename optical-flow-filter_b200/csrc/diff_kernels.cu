@@ -16,6 +16,9 @@
 // they need no atomics and are deterministic; only the coarse-flow gradient of the delta
 // update is scattered with atomics.  Gradients of the per-level scalars are reduced per
 // block, then added once per block.
+//
+// Inputs are plain pointers, not const __restrict__: the kernel before may still be writing them
+// when a kernel starts (ld_waited, launch.cuh).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -216,7 +219,7 @@ __device__ __forceinline__ void put(T& dst, T v) {
 
 // ------------------------------------------------------------------ pyramid (float path)
 template <typename T>
-__global__ void pyr_fwd_k(const T* __restrict__ in, T* __restrict__ out, int H, int W) {
+__global__ void pyr_fwd_k(const T* in, T* __restrict__ out, int H, int W) {
     grid_dep_wait();
     grid_dep_launch();
     const int h = H / 2, w = W / 2;
@@ -236,7 +239,7 @@ __global__ void pyr_fwd_k(const T* __restrict__ in, T* __restrict__ out, int H, 
 // gather form: input pixel (X, Y) sums the contributions of the outputs whose 3x3 stencil
 // (after clamping) reads it; outputs x in [X/2 - 1, X/2 + 1] cover every case
 template <typename T>
-__global__ void pyr_bwd_k(const T* __restrict__ gout, T* gin, int H, int W) {
+__global__ void pyr_bwd_k(const T* gout, T* gin, int H, int W) {
     grid_dep_wait();
     grid_dep_launch();
     const int h = H / 2, w = W / 2;
@@ -262,7 +265,7 @@ __global__ void pyr_bwd_k(const T* __restrict__ gout, T* gin, int H, int W) {
 
 // ------------------------------------------------------------------ image model
 template <typename T>
-__global__ void model_fwd_k(const T* __restrict__ img, T* __restrict__ a0, T* __restrict__ grad, int H, int W) {
+__global__ void model_fwd_k(const T* img, T* __restrict__ a0, T* __restrict__ grad, int H, int W) {
     grid_dep_wait();
     grid_dep_launch();
     PIX_SETUP
@@ -307,7 +310,7 @@ __device__ __forceinline__ T tap_w(const T* w, int i, int j, int n, bool inner) 
 // step 1 (gather): gradients of the Y blur by (used by a0 and ax along X) and of the X blur
 // bx (used by ay along Y) at this pixel
 template <typename T>
-__global__ void model_bwd1_k(const T* __restrict__ ga0, const T* __restrict__ ggrad, T* gby, T* gbx, int H, int W) {
+__global__ void model_bwd1_k(const T* ga0, const T* ggrad, T* gby, T* gbx, int H, int W) {
     grid_dep_wait();
     grid_dep_launch();
     PIX_SETUP
@@ -328,7 +331,7 @@ __global__ void model_bwd1_k(const T* __restrict__ ga0, const T* __restrict__ gg
 
 // step 2 (gather): by = Y blur of the image, bx = X blur of the image
 template <typename T, bool ACC = true>
-__global__ void model_bwd2_k(const T* __restrict__ gby, const T* __restrict__ gbx, T* gimg, int H, int W) {
+__global__ void model_bwd2_k(const T* gby, const T* gbx, T* gimg, int H, int W) {
     grid_dep_wait();
     grid_dep_launch();
     PIX_SETUP
@@ -344,7 +347,7 @@ __global__ void model_bwd2_k(const T* __restrict__ gby, const T* __restrict__ gb
 
 // ------------------------------------------------------------------ propagation sub-step
 template <typename T, int AXIS, bool PAYLOAD>
-__global__ void prop_fwd_k(const T* __restrict__ f, const T* __restrict__ s, const T* __restrict__ v, T* __restrict__ fo,
+__global__ void prop_fwd_k(const T* f, const T* s, const T* v, T* __restrict__ fo,
                            T* __restrict__ so, T* __restrict__ vo, int H, int W, T dt, int border) {
     grid_dep_wait();
     grid_dep_launch();
@@ -459,7 +462,7 @@ __device__ __forceinline__ void prop_adj_at(int j, int n, bool line_in, int bord
 
 // every channel of one pixel of a propagated field (f pairs, s scalars, v pairs) at index k
 template <typename T, bool PAYLOAD>
-__device__ __forceinline__ void field_px(const T* __restrict__ f, const T* __restrict__ s, const T* __restrict__ v,
+__device__ __forceinline__ void field_px(const T* f, const T* s, const T* v,
                                          size_t k, T (&o)[PAYLOAD ? 5 : 2]) {
     const auto a = ld2(f, k);
     o[0] = a.x;
@@ -474,8 +477,8 @@ __device__ __forceinline__ void field_px(const T* __restrict__ f, const T* __res
 
 // Adjoint of one upwind sub-step, one thread per input pixel (prop_adj_at over global memory)
 template <typename T, int AXIS, bool PAYLOAD, bool ACC = true>
-__global__ void prop_bwd_k(const T* __restrict__ f, const T* __restrict__ s, const T* __restrict__ v,
-                           const T* __restrict__ gfo, const T* __restrict__ gso, const T* __restrict__ gvo, T* gf, T* gs,
+__global__ void prop_bwd_k(const T* f, const T* s, const T* v,
+                           const T* gfo, const T* gso, const T* gvo, T* gf, T* gs,
                            T* gv, int H, int W, T dt, int border) {
     grid_dep_wait();
     grid_dep_launch();
@@ -502,8 +505,8 @@ __global__ void prop_bwd_k(const T* __restrict__ f, const T* __restrict__ s, con
 
 // ------------------------------------------------------------------ update (top level)
 template <typename T>
-__global__ void update_fwd_k(const T* __restrict__ a0, const T* __restrict__ grad, const T* __restrict__ old,
-                             const T* __restrict__ fh, const T* __restrict__ gamma, T* __restrict__ out, int H, int W,
+__global__ void update_fwd_k(const T* a0, const T* grad, const T* old,
+                             const T* fh, const T* gamma, T* __restrict__ out, int H, int W,
                              T maxflow) {
     grid_dep_wait();
     grid_dep_launch();
@@ -522,8 +525,8 @@ __device__ __forceinline__ bool passes(T o, T m) {
 }
 
 template <typename T>
-__global__ void update_bwd_k(const T* __restrict__ a0, const T* __restrict__ grad, const T* __restrict__ old,
-                             const T* __restrict__ fh, const T* __restrict__ gamma, const T* __restrict__ gout, T* ga0,
+__global__ void update_bwd_k(const T* a0, const T* grad, const T* old,
+                             const T* fh, const T* gamma, const T* gout, T* ga0,
                              T* ggrad, T* gold, T* gfh, T* ggamma, int H, int W, T maxflow) {
     grid_dep_wait();
     grid_dep_launch();
@@ -551,8 +554,8 @@ __global__ void update_bwd_k(const T* __restrict__ a0, const T* __restrict__ gra
 
 // ------------------------------------------------------------------ delta update
 template <typename T>
-__global__ void dupdate_fwd_k(const T* __restrict__ a0, const T* __restrict__ grad, const T* __restrict__ old,
-                              const T* __restrict__ dh, const T* __restrict__ coarse, const T* __restrict__ gamma,
+__global__ void dupdate_fwd_k(const T* a0, const T* grad, const T* old,
+                              const T* dh, const T* coarse, const T* gamma,
                               T* __restrict__ flow, T* __restrict__ delta, int H, int W, int Hc, int Wc, T maxflow) {
     grid_dep_wait();
     grid_dep_launch();
@@ -571,9 +574,9 @@ __global__ void dupdate_fwd_k(const T* __restrict__ a0, const T* __restrict__ gr
 }
 
 template <typename T>
-__global__ void dupdate_bwd_k(const T* __restrict__ a0, const T* __restrict__ grad, const T* __restrict__ old,
-                              const T* __restrict__ dh, const T* __restrict__ coarse, const T* __restrict__ gamma,
-                              const T* __restrict__ gflow, const T* __restrict__ gdelta, T* ga0, T* ggrad, T* gold,
+__global__ void dupdate_bwd_k(const T* a0, const T* grad, const T* old,
+                              const T* dh, const T* coarse, const T* gamma,
+                              const T* gflow, const T* gdelta, T* ga0, T* ggrad, T* gold,
                               T* gdh, T* gcoarse, T* ggamma, int H, int W, int Hc, int Wc, T maxflow) {
     grid_dep_wait();
     grid_dep_launch();
@@ -610,7 +613,7 @@ __global__ void dupdate_bwd_k(const T* __restrict__ a0, const T* __restrict__ gr
 
 // ------------------------------------------------------------------ weighted smoothing pass
 template <typename T, int AXIS>
-__global__ void smooth_fwd_k(const T* __restrict__ w5, const T* __restrict__ in, T* __restrict__ out, int H, int W,
+__global__ void smooth_fwd_k(const T* w5, const T* in, T* __restrict__ out, int H, int W,
                              T* __restrict__ out2 = nullptr) {
     grid_dep_wait();
     grid_dep_launch();
@@ -635,7 +638,7 @@ __global__ void smooth_fwd_k(const T* __restrict__ w5, const T* __restrict__ in,
 // PART: gw5 is a partial-sum array, this block stores its 5 sums at gw5[5 * block]
 constexpr int kSmoothRows = 4;
 template <typename T, int AXIS, bool ACC = true, bool PART = false>
-__global__ void smooth_bwd_k(const T* __restrict__ w5, const T* __restrict__ in, const T* __restrict__ gout, T* gin,
+__global__ void smooth_bwd_k(const T* w5, const T* in, const T* gout, T* gin,
                              T* gw5, int H, int W) {
     grid_dep_wait();
     grid_dep_launch();
@@ -705,9 +708,9 @@ constexpr size_t smooth_iter_smem() {
 }
 // G2: a second output gradient gout2 is added to gout (image b at gout2 + b * g2_bstride)
 template <typename T, bool ACC, bool G2>
-__global__ void __launch_bounds__(256) smooth_iter_bwd_k(const T* __restrict__ w5, const T* __restrict__ xin,
-                                                         const T* __restrict__ xmid, const T* __restrict__ gout,
-                                                         const T* __restrict__ gout2, long long g2_bstride,
+__global__ void __launch_bounds__(256) smooth_iter_bwd_k(const T* w5, const T* xin,
+                                                         const T* xmid, const T* gout,
+                                                         const T* gout2, long long g2_bstride,
                                                          T* __restrict__ gin, T* __restrict__ part, int H, int W) {
     grid_dep_wait();
     using V = typename Pair<T>::V;
@@ -947,9 +950,9 @@ struct UpwindAdj {
 // pixel per lane and more warps: 27.8 and 30.3 us.
 template <typename T, bool PAYLOAD, bool ACC, bool CLAMP>
 __global__ void __launch_bounds__(32 * kPropWarps)
-    prop_iter_bwd_k(const T* __restrict__ xf, const T* __restrict__ xs, const T* __restrict__ xv,
-                    const T* __restrict__ yf, const T* __restrict__ ys, const T* __restrict__ yv,
-                    const T* __restrict__ gfo, const T* __restrict__ gso, const T* __restrict__ gvo,
+    prop_iter_bwd_k(const T* xf, const T* xs, const T* xv,
+                    const T* yf, const T* ys, const T* yv,
+                    const T* gfo, const T* gso, const T* gvo,
                     T* __restrict__ gf, T* __restrict__ gs, T* __restrict__ gv, int H, int W, T dt, int border, int nwx,
                     int bands, int rows, int warps, bool vec) {
     using R = PropRow<T, PAYLOAD>;
@@ -1136,7 +1139,7 @@ constexpr size_t model_tile_smem() {
     return sizeof(T) * (size_t)(kSW * kSW + 2 * kSW * kSW + 2 * kST * kSW);
 }
 template <typename T, bool ACC>
-__global__ void __launch_bounds__(256) model_tile_bwd_k(const T* __restrict__ ga0, const T* __restrict__ ggrad,
+__global__ void __launch_bounds__(256) model_tile_bwd_k(const T* ga0, const T* ggrad,
                                                         T* __restrict__ gimg, int H, int W) {
     grid_dep_wait();
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1261,8 +1264,8 @@ struct FrameAdj {
 };
 
 template <typename T>
-__global__ void update_bwd_frame_k(const T* __restrict__ a0, const T* __restrict__ grad, const T* __restrict__ old,
-                                   const T* __restrict__ fh, const T* __restrict__ gamma, const T* __restrict__ gout,
+__global__ void update_bwd_frame_k(const T* a0, const T* grad, const T* old,
+                                   const T* fh, const T* gamma, const T* gout,
                                    T* ga0, T* ggrad, T* gold, T* gfh, FrameAdj<T> fa, int H, int W, T maxflow) {
     grid_dep_wait();
     grid_dep_launch();
@@ -1283,10 +1286,10 @@ __global__ void update_bwd_frame_k(const T* __restrict__ a0, const T* __restrict
 }
 
 template <typename T>
-__global__ void dupdate_bwd_frame_k(const T* __restrict__ a0, const T* __restrict__ grad, const T* __restrict__ old,
-                                    const T* __restrict__ dh, const T* __restrict__ coarse,
-                                    const T* __restrict__ gamma, const T* __restrict__ gflow,
-                                    const T* __restrict__ gdelta, T* ga0, T* ggrad, T* gold, T* gdh, T* gcoarse,
+__global__ void dupdate_bwd_frame_k(const T* a0, const T* grad, const T* old,
+                                    const T* dh, const T* coarse,
+                                    const T* gamma, const T* gflow,
+                                    const T* gdelta, T* ga0, T* ggrad, T* gold, T* gdh, T* gcoarse,
                                     FrameAdj<T> fa, int H, int W, int Hc, int Wc, T maxflow) {
     grid_dep_wait();
     grid_dep_launch();
@@ -1339,7 +1342,7 @@ __global__ void dupdate_bwd_frame_k(const T* __restrict__ a0, const T* __restric
 
 // dst[v] += sum over i < n of part[i * NV + v], one block (fixed order: deterministic)
 template <typename T, int NV>
-__global__ void reduce_parts_k(const T* __restrict__ part, int n, T* dst) {
+__global__ void reduce_parts_k(const T* part, int n, T* dst) {
     grid_dep_wait();
     grid_dep_launch();
     T acc[NV];
@@ -1386,7 +1389,7 @@ __global__ void __launch_bounds__(1024) reduce_jobs_k(ReduceJobs<T> J) {
 // dst = (ACC ? dst : 0) + a + b over B images of `per` elements; a dense (nullable, zero),
 // image i of b at b + i * bstride
 template <typename T, bool ACC>
-__global__ void sum2_k(T* __restrict__ dst, const T* __restrict__ a, const T* __restrict__ b, long long bstride,
+__global__ void sum2_k(T* __restrict__ dst, const T* a, const T* b, long long bstride,
                        long long per, int B) {
     grid_dep_wait();
     grid_dep_launch();
@@ -1400,7 +1403,7 @@ __global__ void sum2_k(T* __restrict__ dst, const T* __restrict__ a, const T* __
 
 // dst += src over n elements
 template <typename T>
-__global__ void add_k(T* __restrict__ dst, const T* __restrict__ src, size_t n) {
+__global__ void add_k(T* __restrict__ dst, const T* src, size_t n) {
     grid_dep_wait();
     grid_dep_launch();
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
@@ -1419,7 +1422,7 @@ struct EpeGeom {
 };
 constexpr int kEpeThreads = 256, kEpeBlocks = 1024;
 template <typename T>
-__global__ void __launch_bounds__(kEpeThreads) epe_fwd_k(const T* __restrict__ flows, const T* __restrict__ truth,
+__global__ void __launch_bounds__(kEpeThreads) epe_fwd_k(const T* flows, const T* truth,
                                                          EpeGeom g, T eps, T* __restrict__ part) {
     grid_dep_wait();
     grid_dep_launch();
@@ -1436,7 +1439,7 @@ __global__ void __launch_bounds__(kEpeThreads) epe_fwd_k(const T* __restrict__ f
     block_sum<T, 1>(acc, part + blockIdx.x, false);
 }
 template <typename T>
-__global__ void __launch_bounds__(1024) epe_sum_k(const T* __restrict__ part, int n, T inv_count, T* loss) {
+__global__ void __launch_bounds__(1024) epe_sum_k(const T* part, int n, T inv_count, T* loss) {
     grid_dep_wait();
     grid_dep_launch();
     T acc[1] = {T(0)};
@@ -1447,8 +1450,8 @@ __global__ void __launch_bounds__(1024) epe_sum_k(const T* __restrict__ part, in
     if (threadIdx.x == 0) *loss = tot[0] * inv_count;
 }
 template <typename T>
-__global__ void __launch_bounds__(kEpeThreads) epe_bwd_k(const T* __restrict__ flows, const T* __restrict__ truth,
-                                                         EpeGeom g, T eps, const T* __restrict__ gloss, T inv_count,
+__global__ void __launch_bounds__(kEpeThreads) epe_bwd_k(const T* flows, const T* truth,
+                                                         EpeGeom g, T eps, const T* gloss, T inv_count,
                                                          T* __restrict__ gflows) {
     grid_dep_wait();
     grid_dep_launch();

@@ -42,8 +42,8 @@ __device__ __forceinline__ int wheel_texel(float f, float m) {
     return (int)__fmul_rn(u, (float)kWheel);
 }
 
-__global__ void flow_to_color_k(const float* __restrict__ flow, size_t flow_pitch, int H, int W, float maxflow,
-                                const uchar4* __restrict__ wheel, uchar4* __restrict__ color, size_t color_pitch) {
+__global__ void flow_to_color_k(const float* flow, size_t flow_pitch, int H, int W, float maxflow,
+                                const uchar4* wheel, uchar4* __restrict__ color, size_t color_pitch) {
     grid_dep_wait();
     grid_dep_launch();
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
@@ -51,7 +51,7 @@ __global__ void flow_to_color_k(const float* __restrict__ flow, size_t flow_pitc
     if (x >= W || y >= H) return;
     const float2 f = reinterpret_cast<const float2*>(reinterpret_cast<const char*>(flow) + y * flow_pitch)[x];
     const uchar4* w = wheel ? wheel : g_default_wheel;
-    const uchar4 c = __ldg(&w[wheel_texel(f.y, maxflow) * kWheel + wheel_texel(f.x, maxflow)]);
+    const uchar4 c = w[wheel_texel(f.y, maxflow) * kWheel + wheel_texel(f.x, maxflow)];
     reinterpret_cast<uchar4*>(reinterpret_cast<char*>(color) + y * color_pitch)[x] = c;
 }
 

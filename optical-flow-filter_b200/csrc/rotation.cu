@@ -161,36 +161,45 @@ __global__ void __launch_bounds__(32 * kWarps) lw_rows_k(LWArgs a, int nwx, int 
         pxa = __fdiv_rn(__fsub_rn((float)ca, a.cx), a.ax);
         pxb = __fdiv_rn(__fsub_rn((float)cb, a.cx), a.ax);
     }
-    for (int y = sy0 + warp; y < sy1; y += kWarps) {
-        char* row = smem + (y - sy0) * ROWB;
+    // a row ahead of its use (plain loads: the kernel before may have written image and flow)
+    Pix2<D> v;
+    float2 fa = make_float2(0.f, 0.f), fb = fa;
+    auto fetch = [&](int y) {
+        y = min(y, sy1 - 1);
         const float* srow = reinterpret_cast<const float*>(reinterpret_cast<const char*>(a.src) + y * a.src_pitch);
-        Pix2<D> v;
         if constexpr (D == 4) {
-            const float4 q = __ldg(reinterpret_cast<const float4*>(srow) + ca), r = __ldg(reinterpret_cast<const float4*>(srow) + cb);
+            const float4 q = reinterpret_cast<const float4*>(srow)[ca], r = reinterpret_cast<const float4*>(srow)[cb];
             v.a[0] = q.x, v.a[1] = q.y, v.a[2] = q.z, v.a[3] = q.w;
             v.b[0] = r.x, v.b[1] = r.y, v.b[2] = r.z, v.b[3] = r.w;
         } else {
-            v.a[0] = __ldg(srow + ca);
-            v.b[0] = __ldg(srow + cb);
+            v.a[0] = srow[ca];
+            v.b[0] = srow[cb];
         }
-        float2 fa, fb;
+        if (!ROT) {
+            const float2* frow = reinterpret_cast<const float2*>(reinterpret_cast<const char*>(a.flow) + y * a.flow_pitch);
+            fa = frow[ca];
+            fb = frow[cb];
+        }
+    };
+    fetch(sy0 + warp);
+    for (int y = sy0 + warp; y < sy1; y += kWarps) {
+        char* row = smem + (y - sy0) * ROWB;
+        const Pix2<D> w = v;
+        float2 wa = fa, wb = fb;
+        fetch(y + kWarps);
         if (ROT) {
             const float py = __fdiv_rn(__fsub_rn((float)y, a.cy), a.ay);
-            fa = rotational_flow(a, ca, y, pxa, py);
-            fb = rotational_flow(a, cb, y, pxb, py);
+            wa = rotational_flow(a, ca, y, pxa, py);
+            wb = rotational_flow(a, cb, y, pxb, py);
             if (y >= ys && y < ye) {
                 float2* frow = reinterpret_cast<float2*>(reinterpret_cast<char*>(a.flow_out) + y * a.flow_out_pitch);
-                if (nout > 0) frow[c0] = fa;
-                if (nout > 1) frow[c0 + 1] = fb;
+                if (nout > 0) frow[c0] = wa;
+                if (nout > 1) frow[c0 + 1] = wb;
             }
-        } else {
-            const float2* frow = reinterpret_cast<const float2*>(reinterpret_cast<const char*>(a.flow) + y * a.flow_pitch);
-            fa = __ldg(frow + ca);
-            fb = __ldg(frow + cb);
         }
-        sts<D>(row, lane, v);
-        reinterpret_cast<float4*>(row + IMG)[lane] = make_float4(__fmul_rn(a.dt, fa.x), __fmul_rn(a.dt, fa.y),
-                                                                 __fmul_rn(a.dt, fb.x), __fmul_rn(a.dt, fb.y));
+        sts<D>(row, lane, w);
+        reinterpret_cast<float4*>(row + IMG)[lane] = make_float4(__fmul_rn(a.dt, wa.x), __fmul_rn(a.dt, wa.y),
+                                                                 __fmul_rn(a.dt, wb.x), __fmul_rn(a.dt, wb.y));
     }
     grid_dep_launch();
     __syncthreads();

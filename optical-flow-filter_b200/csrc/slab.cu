@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) smooth_slab_k(LevelArgs a, Geo
 // The image model stage alone (ImageModel): a warp takes a 128-column window of `rows` rows, the
 // vertical windows in registers; only 4-column halos and 4 rows per run are computed twice.
 template <typename P>
-__global__ void __launch_bounds__(32 * kWarps) image_model_rows_k(const P* __restrict__ img, size_t pitch, int H, int W,
+__global__ void __launch_bounds__(32 * kWarps) image_model_rows_k(const P* img, size_t pitch, int H, int W,
                                                                  float* __restrict__ a0, size_t a0_pitch,
                                                                  float2* __restrict__ grad, size_t grad_pitch, int nwx,
                                                                  int rows) {
@@ -121,16 +121,16 @@ __global__ void __launch_bounds__(32 * kWarps) image_model_rows_k(const P* __res
         float v[4];
         if constexpr (sizeof(P) == 1) {
             uint32_t q;
-            if (word) q = __ldg(reinterpret_cast<const uint32_t*>(r + c.c0));
-            else q = __ldg(r + o[0]) | __ldg(r + o[1]) << 8 | __ldg(r + o[2]) << 16 | (uint32_t)__ldg(r + o[3]) << 24;
+            if (word) q = ld_waited(reinterpret_cast<const uint32_t*>(r + c.c0));
+            else q = r[o[0]] | r[o[1]] << 8 | r[o[2]] << 16 | (uint32_t)r[o[3]] << 24;
 #pragma unroll
             for (int j = 0; j < 4; ++j) v[j] = u8_to_unit((q >> (8 * j)) & 0xffu);
         } else if (word) {
-            const float4 q = __ldg(reinterpret_cast<const float4*>(r + c.c0));
+            const float4 q = ld_waited(reinterpret_cast<const float4*>(r + c.c0));
             v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
         } else {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) v[j] = __ldg(r + o[j]);
+            for (int j = 0; j < 4; ++j) v[j] = ld_waited(r + o[j]);
         }
         return Q{make_float2(v[0], v[1]), make_float2(v[2], v[3])};
     };

@@ -61,11 +61,11 @@ __global__ void __launch_bounds__(BX * BY) pyramid_down2_k(CView<P> in, View<P> 
                 const uint8_t* row = reinterpret_cast<const uint8_t*>(in.row(min(max(Y0 + r, 0), H - 1)));
                 const int x = X0 + 4 * c;
                 if (x >= 0 && x + 3 < W) {
-                    v[u] = __ldg(reinterpret_cast<const uint32_t*>(row + x));
+                    v[u] = *reinterpret_cast<const uint32_t*>(row + x);
                 } else {  // a word beyond an edge: its clamped pixels
                     uint32_t w = 0;
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) w |= (uint32_t)__ldg(row + min(max(x + q, 0), W - 1)) << (8 * q);
+                    for (int q = 0; q < 4; ++q) w |= (uint32_t)row[min(max(x + q, 0), W - 1)] << (8 * q);
                     v[u] = w;
                 }
             }
