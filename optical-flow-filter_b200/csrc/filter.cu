@@ -350,12 +350,13 @@ bool Filter::any_first() const {
 }
 
 void Filter::batch_begin(cudaStream_t s) {
-    if (ops_ != batch_seen_) begin_on(s);
+    if (ops_ != batch_seen_ || s != batch_stream_) begin_on(s);
 }
 
 void Filter::batch_end(cudaStream_t s) {
     end_on(s);
     batch_seen_ = ops_;
+    batch_stream_ = s;
     cur_ ^= 1;
     for (Level& v : lv_) v.first = false;
     phase_ = 0;

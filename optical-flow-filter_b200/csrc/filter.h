@@ -198,7 +198,8 @@ public:
     void wait_done() const;
     // changes whenever a parameter that shapes the level steps changes
     unsigned long long config_generation() const { return config_gen_; }
-    // order stream s after this filter's own work queued since the last batch step
+    // order stream s after this filter's work: its own since the last batch step, and that step
+    // where it ran on another stream
     void batch_begin(cudaStream_t s);
     // a batch finished this filter's frame on s: record it and advance the state parity
     void batch_end(cudaStream_t s);
@@ -246,6 +247,7 @@ private:
     unsigned long long config_gen_ = 0;  // bumped by drop_graphs (every parameter change)
     unsigned long long ops_ = 0;         // bumped by end_on
     unsigned long long batch_seen_ = 0;  // ops_ after the last batch step
+    cudaStream_t batch_stream_ = nullptr;  // the stream of that step
     cudaGraphExec_t graph_exec_[2] = {nullptr, nullptr};
     int prof_cap_ = 0, prof_count_ = 0;
     std::vector<cudaEvent_t> prof_ev_;
