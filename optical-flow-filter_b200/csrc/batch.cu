@@ -269,12 +269,16 @@ tile::Geom batch_geom(bool delta, int N, int S, int W, int H, size_t* smem) {
     return best;
 }
 
+// a table in device memory, in place when this returns: uploaded on s, a stream that the
+// default stream's work does not hold up, and waited for there (a copy from pageable memory may
+// return before it has arrived, and the step's stream is not ordered after the default stream)
 template <typename T>
-T* to_device(const std::vector<T>& v) {
+T* to_device(const std::vector<T>& v, cudaStream_t s) {
     if (v.empty()) return nullptr;
     T* d = nullptr;
     check_cuda(device_malloc((void**)&d, v.size() * sizeof(T)), "batch tables");
-    const cudaError_t e = cudaMemcpy(d, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice);
+    cudaError_t e = cudaMemcpyAsync(d, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) cudaFree(d);
     check_cuda(e, "batch tables");
     return d;
@@ -356,14 +360,14 @@ void Batch::init(int n, const int* heights, const int* widths, const int* levels
         blocks += j.tiles_x * j.tiles_y;
         ing.push_back(j);
     }
-    d_ingest_ = to_device(ing);
+    d_ingest_ = to_device(ing, cap_);
     ingest_blocks_ = blocks;
     if (n > 65535) throw Error(FF_ERR_UNSUPPORTED, "batch: at most 65535 streams");
     std::vector<unsigned short> block_job(blocks);
     for (int i = 0; i < n; ++i)
         for (int b = ing[i].first_block; b < ing[i].first_block + ing[i].tiles_x * ing[i].tiles_y; ++b)
             block_job[b] = (unsigned short)i;
-    d_ingest_block_ = to_device(block_job);
+    d_ingest_block_ = to_device(block_job, cap_);
     for (auto& t : tab_) t.reset(new Table);
     check_cuda(cudaFuncSetAttribute(tile_batch_k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBatchSmemCap),
                "cudaFuncSetAttribute");
@@ -694,9 +698,9 @@ void Batch::build(Table& t) {
     sall.insert(sall.end(), sj[1].begin(), sj[1].end());
     std::vector<TileJob> tall(tj[0]);
     tall.insert(tall.end(), tj[1].begin(), tj[1].end());
-    t.d_pyr = to_device(pyr);
-    t.d_tile = to_device(tall);
-    t.d_stream = to_device(sall);
+    t.d_pyr = to_device(pyr, cap_);
+    t.d_tile = to_device(tall, cap_);
+    t.d_stream = to_device(sall, cap_);
     std::vector<SlabJob> slall;
     size_t slfirst[2][2] = {};
     for (int ph = 0; ph < 2; ++ph)
@@ -704,7 +708,7 @@ void Batch::build(Table& t) {
             slfirst[ph][k] = slall.size();
             slall.insert(slall.end(), sl[ph][k].begin(), sl[ph][k].end());
         }
-    t.d_slab = to_device(slall);
+    t.d_slab = to_device(slall, cap_);
     t.parity.clear();
     t.gen.clear();
     for (auto& f : f_) {

@@ -170,6 +170,8 @@ ff_status ff_memcpy2d(void* dst, size_t dpitch, const void* src, size_t spitch, 
                                        : cudaMemcpyDefault;
         if (kind < 0 || kind > 2) throw Error(FF_ERR_INVALID_ARGUMENT, "copy kind must be 0, 1 or 2");
         ffb::check_cuda(cudaMemcpy2D(dst, dpitch, src, spitch, width_bytes, height, k), "cudaMemcpy2D");
+        // copies to the device may still be on their way, and filters run on streams of their own
+        if (kind != 1) ffb::check_cuda(cudaStreamSynchronize(nullptr), "cudaMemcpy2D");
     });
 }
 
@@ -177,6 +179,7 @@ ff_status ff_memset2d(void* dptr, size_t pitch, int value, size_t width_bytes, s
     return guard([&] {
         need(dptr, "pointer");
         ffb::check_cuda(cudaMemset2D(dptr, pitch, value, width_bytes, height), "cudaMemset2D");
+        ffb::check_cuda(cudaStreamSynchronize(nullptr), "cudaMemset2D");  // as after a copy
     });
 }
 

@@ -72,6 +72,7 @@ cudaError_t ensure_default_wheel() {
     if ((int)done.size() <= dev) done.resize(dev + 1, false);
     if (done[dev]) return cudaSuccess;
     e = cudaMemcpyToSymbol(g_default_wheel, default_wheel().data(), default_wheel().size());
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);  // in place before any stream reads it
     if (e == cudaSuccess) done[dev] = true;
     return e;
 }
