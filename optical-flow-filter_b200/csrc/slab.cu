@@ -236,6 +236,14 @@ cudaError_t set_access(bool delta, LevelArgs& a) {
     return cudaSuccess;
 }
 
+// The same for fields of a caller: rows4 counts on the padding after a row's last pixel, which
+// after the last row is not the caller's to read
+cudaError_t set_access_of_caller(bool delta, LevelArgs& a) {
+    const cudaError_t e = set_access(delta, a);
+    a.vec = a.vec && a.W % 4 == 0;
+    return e;
+}
+
 // once per kernel and device: the shared-memory limit, and the full shared carve-out as for the
 // tile kernels (SMs running small slabs can then also host the other levels' kernels)
 template <auto* K>
@@ -266,7 +274,7 @@ cudaError_t launch(LevelArgs a, int N, int S, cudaStream_t s) {
 
 template <bool DELTA>
 cudaError_t launch_propagate_slab(LevelArgs a, int N, cudaStream_t s) {
-    cudaError_t e = set_access(DELTA, a);
+    cudaError_t e = set_access_of_caller(DELTA, a);
     if (e == cudaSuccess) e = prepare<propagate_slab_k<DELTA>>();
     if (e != cudaSuccess) return e;
     const Geom g = auto_geom(DELTA, N, 0, a.W, a.H, 1);
@@ -409,7 +417,7 @@ cudaError_t launch_smooth_stage(const float* flow, size_t fp, int H, int W, int 
     a.W = W;
     a.fs_in = flow, a.fs_in_pitch = fp;
     a.fs_out = out, a.fs_out_pitch = op;
-    cudaError_t e = slab::set_access(false, a);
+    cudaError_t e = slab::set_access_of_caller(false, a);
     if (e == cudaSuccess) e = slab::prepare<slab::smooth_slab_k>();
     if (e != cudaSuccess) return e;
     const slab::Geom g = slab::auto_geom(false, 0, S, W, H, 1);
