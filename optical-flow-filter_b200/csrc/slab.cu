@@ -281,11 +281,15 @@ cudaError_t launch_propagate_slab(LevelArgs a, int N, cudaStream_t s) {
     return launch_k(propagate_slab_k<DELTA>, dim3(g.slabs(a.H)), dim3(32 * kWarps), smem_of(DELTA, g), s, a, g);
 }
 
-// the rows [p, p + pitch * H) of two fields share memory
-bool overlap(const void* a, size_t ap, const void* b, size_t bp, int H) {
-    const char *x = (const char*)a, *y = (const char*)b;
-    return x < y + bp * H && y < x + ap * H;
-}
+// the H rows of a field of `row` bytes each, from the first byte of the first to the last of the
+// last (rows may lie closer than their length, or all be one row: pitch 0)
+struct Rows {
+    const void* p;
+    size_t pitch, row;
+    uintptr_t begin() const { return (uintptr_t)p; }
+    uintptr_t end(int H) const { return begin() + (size_t)(H - 1) * pitch + row; }
+};
+bool overlap(const Rows& a, const Rows& b, int H) { return a.begin() < b.end(H) && b.begin() < a.end(H); }
 
 // the most sub-step pairs or smoothing iterations of one slab launch
 constexpr int kMaxFused = 8;
@@ -370,7 +374,7 @@ cudaError_t launch_slab_images(bool delta, int N, int S, int images, const Level
 // one-thread-per-pixel form reads 50 pixels for each
 cudaError_t launch_propagate_stage(const float* flow, size_t fp, int H, int W, int N, int border, float* out, size_t op,
                                    float* tmp, size_t tp, cudaStream_t s) {
-    if (N > slab::kMaxFused || ((fp | op) >> 32) || slab::overlap(flow, fp, out, op, H))
+    if (N > slab::kMaxFused || ((fp | op) >> 32) || slab::overlap({flow, fp, 8 * (size_t)W}, {out, op, 8 * (size_t)W}, H))
         return launch_propagate(flow, fp, H, W, N, border, out, op, tmp, tp, s);
     LevelArgs a{};
     a.H = H;
@@ -385,13 +389,12 @@ cudaError_t launch_propagate_payload_stage(const float* flow, size_t fp, const f
                                            size_t vp, int H, int W, int N, int border, float* of, size_t ofp, float* os,
                                            size_t osp, float* ov, size_t ovp, float* tf, size_t tfp, float* ts, size_t tsp,
                                            float* tv, size_t tvp, cudaStream_t s) {
-    const void* in[3] = {flow, sc, ve};
-    const size_t ip[3] = {fp, sp, vp};
-    const void* out[3] = {of, os, ov};
-    const size_t op[3] = {ofp, osp, ovp};
+    const size_t w = (size_t)W;
+    const slab::Rows in[3] = {{flow, fp, 8 * w}, {sc, sp, 4 * w}, {ve, vp, 8 * w}};
+    const slab::Rows out[3] = {{of, ofp, 8 * w}, {os, osp, 4 * w}, {ov, ovp, 8 * w}};
     bool plain = N > slab::kMaxFused || ((fp | sp | vp | ofp | osp | ovp) >> 32);
-    for (int i = 0; i < 3; ++i)
-        for (int o = 0; o < 3; ++o) plain |= slab::overlap(in[i], ip[i], out[o], op[o], H);
+    for (const slab::Rows& i : in)
+        for (const slab::Rows& o : out) plain |= slab::overlap(i, o, H);
     if (plain)
         return launch_propagate_payload(flow, fp, sc, sp, ve, vp, H, W, N, border, of, ofp, os, osp, ov, ovp, tf, tfp, ts,
                                         tsp, tv, tvp, s);
@@ -410,7 +413,7 @@ cudaError_t launch_propagate_payload_stage(const float* flow, size_t fp, const f
 
 cudaError_t launch_smooth_stage(const float* flow, size_t fp, int H, int W, int S, float* out, size_t op, float* tmp,
                                 size_t tp, cudaStream_t s) {
-    if (S > slab::kMaxFused || ((fp | op) >> 32) || slab::overlap(flow, fp, out, op, H))
+    if (S > slab::kMaxFused || ((fp | op) >> 32) || slab::overlap({flow, fp, 8 * (size_t)W}, {out, op, 8 * (size_t)W}, H))
         return launch_smooth(flow, fp, H, W, S, out, op, tmp, tp, s);
     LevelArgs a{};
     a.H = H;
