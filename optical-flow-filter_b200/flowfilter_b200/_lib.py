@@ -227,11 +227,15 @@ def call(name: str, *args) -> None:
 def current_stream() -> int:
     """The handle of torch's current stream on the current device.  torch.cuda.current_stream()
     builds a Stream object on each call (3.3 us of a small frame's 29); the handle alone takes a
-    tenth of that."""
+    tenth of that, through functions that torch keeps for its own code generators: a torch
+    without them gets the Stream."""
     import torch
 
     if torch.cuda.is_initialized():
-        return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+        try:
+            return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+        except AttributeError:
+            pass
     return torch.cuda.current_stream().cuda_stream
 
 
