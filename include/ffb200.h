@@ -128,10 +128,10 @@ ff_status ff_filter_get_propagation_border(const ff_filter* f, int* border);
 ff_status ff_filter_get_propagation_iterations(const ff_filter* f, int level, int* iterations);
 
 /* Kernel selection per level: 0 per-stage kernels, 1 the streaming fused per-level kernel
- * wherever it is instantiated, 2 automatic (default: the autotuned choice, else by
- * size and smoothing the slab kernel, the streaming kernel for the largest levels or the
- * tile-fused kernel for the smallest delta levels), 3 the tile-fused kernel wherever it fits in shared memory.  All modes give bit-identical
- * results. */
+ * wherever it is instantiated, 2 automatic (default: the autotuned choice, else by size and
+ * iterations the slab kernel, the streaming kernel for the largest levels, the tile-fused
+ * kernel for the smallest ones or the per-stage kernels for many iterations), 3 the tile-fused
+ * kernel wherever it fits in shared memory.  All modes give bit-identical results. */
 ff_status ff_filter_set_fused(ff_filter* f, int mode);
 
 /* Replay the frame step from CUDA graphs (one per state buffer parity, captured on first

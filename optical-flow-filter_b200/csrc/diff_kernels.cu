@@ -2102,8 +2102,14 @@ struct Driver {
         for (int l = 1; l < L; ++l)
             ok(launch_k(pyr_fwd_k<T>, grid3(g.W[l], g.H[l], g.B), kBlock, 0, s, img(l - 1), tp + tape.img[l],
                         g.H[l - 1], g.W[l - 1]));
-        // the float filter's level steps run as one kernel each where the slab kernel covers them
-        auto slab = [&](int l) { return std::is_same<T, float>::value && slab_available(l < top, g.N[l], g.S[l]); };
+        // the float filter's level steps run as one kernel each where the slab kernel covers them and
+        // its halo does not cost more than the launches it saves (device us of a level, slab / stage
+        // kernels: 16 images of 256x256, delta, N 4 S 8 177 / 223, N 8 S 8 292 / 292, N 20 S 8
+        // 1385 / 502, N 10 S 15 4400 / 412)
+        auto slab = [&](int l) {
+            return std::is_same<T, float>::value && slab_available(l < top, g.N[l], g.S[l]) &&
+                   slab_pays(l < top, g.N[l], g.S[l], g.W[l], g.H[l], g.B);
+        };
         // top level: flow propagation, update, smoothing
         if (slab(top)) {
             // the unsmoothed flow: level L-2 reads it from the tape, and the adjoint; a single level

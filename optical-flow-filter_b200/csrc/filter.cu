@@ -772,7 +772,14 @@ int Filter::path_of(int l, int* param) const {
         p = band_;
         return kStream;
     }
-    if ((!v.delta || px >= kSlabMinPixels) && slab_ok(l)) return kSlab;
+    // With more iterations than that the tile kernel, with a quarter of the slab's columns, keeps
+    // small levels a little longer (slab / tile: delta 240x320 N 8 S 4 38.2 / 34.4, 280x400
+    // 40.3 / 38.3; top 120x160 25.9 / 23.9, 150x200 24.9 / 23.9), while its tiles still have a
+    // useful size: beyond a halo of 24 rows it takes up to 30 times the per-stage kernels' time,
+    // and the choice is between those and the slab kernel alone.
+    const bool many = (v.iters > 4 || v.smooth > 4) && v.iters + 2 * v.smooth <= 24;
+    if (px >= (v.delta ? (many ? kSlabMinPixelsMany : kSlabMinPixels) : (many ? kSlabMinTopMany : 0)) && slab_ok(l))
+        return slab_pays(v.delta, v.iters, v.smooth, v.W, v.H, 1) ? kSlab : kPerStage;
     if (tile_ok(l, 0)) return kTile;
     return kPerStage;
 }

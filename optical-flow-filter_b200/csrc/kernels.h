@@ -98,6 +98,8 @@ cudaError_t launch_stream_mega(const StreamJob* jobs, int n, int blocks, int sme
 
 // ---- slab level kernel (slab.cu); LevelArgs::band = output rows of a slab (0 automatic)
 bool slab_available(bool delta, int N, int S);
+// is it the faster choice against the per-stage kernels, for `images` levels of this size at once?
+bool slab_pays(bool delta, int N, int S, int W, int H, int images);
 cudaError_t launch_slab_level(bool delta, int N, int S, const LevelArgs& a, cudaStream_t s);
 // the same step of a batch of float images, every field dense (image after image); coarse_rows
 // may be null.  tape (nullable): where to keep the propagated fields (flow, then for delta

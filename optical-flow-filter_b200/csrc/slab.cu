@@ -2,6 +2,7 @@
 #include "slab.cuh"
 
 #include <atomic>
+#include <cmath>
 
 namespace ffb {
 namespace slab {
@@ -339,6 +340,30 @@ cudaError_t launch_slab_jobs(const SlabJob* jobs, int n, int blocks, size_t smem
 }
 
 bool slab_available(bool delta, int N, int S) { return N >= 1 && S >= 1 && slab::max_rows(delta, N, S) >= 1; }
+
+// A slab works on N + 2S more rows on each side than it has, and the most rows it can have fall
+// with them: at N 10, S 15 two of 82.  Estimated times (us) of its stages over the rows of each,
+// and of the 2 + 2N + 2S per-stage launches, which go through memory but work on no pixel twice;
+// fitted on a B200 to 200 levels of 120x160 to 1088x2048, N 1..36, S 1..20 (beyond 20 halo rows
+// the medians are 6% and 5% off, and the worst choice takes 1.15 times the other one).  Measured,
+// us, slab / per-stage: delta levels of 720x1280 N 8 S 8 186 / 218, N 10 S 8 221 / 246, N 10 S 12
+// 579 / 282, N 10 S 15 4354 / 310; top levels N 4 S 12 106 / 166, N 10 S 12 243 / 216, N 28 S 12
+// 19906 / 368.  Halos of up to 20 rows always pay (0.86 of the per-stage time at the most).
+bool slab_pays(bool delta, int N, int S, int W, int H, int images) {
+    const int R = N + 2 * S;
+    if (R <= 20) return true;
+    const slab::Geom g = slab::auto_geom(delta, N, S, W, H, images);
+    const double sms = slab::sm_count(), waves = std::ceil((double)g.slabs(H) * images / sms);
+    auto rows = [&](int r) { return (double)std::min(g.rows + 2 * r, H); };
+    // instructions of a 128-column row: a sub-step pair, model and update, a smoothing iteration
+    double work = 330.0 * rows(2 * S);
+    for (int k = 1; k <= N; ++k) work += (delta ? 185.0 : 80.0) * rows(R - k);
+    for (int s = 1; s <= S; ++s) work += 110.0 * rows(2 * (S - s) + 1);
+    const double slab_us = 14.5 + waves * (3.23e-4 * work + 0.88 * N + 0.24 * S - 5.6);
+    const double mpx = 1e-6 * W * H * images, pass = 1.0 + 3.5 * mpx;
+    const double stage_us = 7.7 + (delta ? 33.4 : 27.0) * mpx + 2 * N * (delta ? 1.76 + 6.13 * mpx : pass) + 2 * S * pass;
+    return slab_us <= stage_us;
+}
 
 cudaError_t launch_slab_level(bool delta, int N, int S, const LevelArgs& a, cudaStream_t s) {
     if (!slab_available(delta, N, S)) return cudaErrorInvalidConfiguration;

@@ -232,9 +232,9 @@ class _FilterBase:
 
     def setFused(self, mode) -> None:
         """Kernel selection: False/0 per-stage kernels, True/1 streaming fused per-level kernels,
-        2 automatic (the default: the autotuned choice, else by size and smoothing the slab
-        kernel, the streaming kernel for the largest levels or the tile-fused kernel for the
-        smallest delta levels), 3 tile-fused kernels.
+        2 automatic (the default: the autotuned choice, else by size and iterations the slab
+        kernel, the streaming kernel for the largest levels, the tile-fused kernel for the
+        smallest ones or the per-stage kernels for many iterations), 3 tile-fused kernels.
         Results are identical."""
         call("ff_filter_set_fused", self._h, int(mode))
 
