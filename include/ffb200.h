@@ -297,7 +297,8 @@ ff_status ff_batch_step(ff_batch* batch, const void* frames, void* stream);
  * previous frame's coarse flow or are top levels (phase A) run the tile-fused kernel below
  * min_pixels pixels (< 0: the slab kernel below 200000), every other level the streaming level kernel covers runs
  * it, in bands of band rows (<= 0: the default rule).  With min_pixels < 0, band <= 0 and no
- * level band set, as at the start, a phase whose levels sum to fewer than 8,000,000 pixels runs
+ * level band set, as at the start, a phase whose levels sum to fewer than 0.5 + 2.5 S million
+ * pixels (S: their smoothing iterations, averaged over the pixels; 8 million at the most) runs
  * them all by the slab kernel instead.  Phase-B levels beyond the streaming
  * kernel (more than 4 iterations or smoothing passes) add a second tile launch. */
 ff_status ff_batch_set_tuning(ff_batch* batch, long long min_pixels, int band);

@@ -433,24 +433,29 @@ bool Batch::slab_beside(const Filter& f, int l) const {
     return min_px_ < 0 && !(L >= 2 && l == L - 2) && !streamed(f, l) && f.slab_usable(l);
 }
 
-// Levels of phase A (0: tops and levels 0..L-3) or phase B (1: levels L-2).  Below kSlabBelow
-// pixels a phase's streaming warps are too few or their bands too short.  Measured step times (us,
-// slab / streaming and tile): 4 streams of 640x480, 2 levels (1.2 M pixels) 91 / 125; 16 of them
-// (4.9 M) 303 / 344; 8 of 1280x720 with 3 levels (7.4 M) 471 / 497; 16 of them (14.7 M) 888 / 785;
-// the 64-stream mix of 54 M pixels 2349 / 2107.
+// Levels of phase A (0: tops and levels 0..L-3) or phase B (1: levels L-2).  In a phase of few
+// pixels the streaming warps are too few or their bands too short; how few depends on the smoothing
+// iterations S, which the streaming kernel's chain per row grows with: below 0.5 + 2.5 S million
+// pixels (S averaged over the phase's pixels), 8 million at the most.  Measured step times, slab /
+// streaming: phase B of 640x480 streams with 2 levels at 2.5, 4.0, 6.1 and 8.0 M pixels, S 1 0.96,
+// 1.04, 1.11, 1.12; S 2 0.88, 0.96, 1.00, 1.03; S 3 0.79, 0.88, 0.90, 0.92; phase A of 640x480
+// streams with one level S 1 0.95, 1.06, 1.14, 1.04, S 2 0.84, 0.94, 0.94, 0.95; of 1920x1080
+// streams with 3 levels at 4.4 and 8.8 M S 1 1.00, 1.10, S 3 0.95, 1.01; 15.7 M and more 1.0 to 1.3.
+// Levels that cannot stream count as S 4: their other kernel, the tile kernel, takes twice as long.
 bool Batch::slab_phase(int phase) const {
     if (min_px_ >= 0 || band_ > 0 || !level_band_.empty()) return false;
-    long px = 0;
+    double px = 0, spx = 0;
     for (auto& f : f_) {
         const int L = f->levels();
         for (int l = 0; l < L; ++l) {
             if ((L >= 2 && l == L - 2) != (phase == 1)) continue;
             const Level& v = f->level(l);
-            px += (long)v.H * v.W;
-            if (px >= kSlabBelow || !f->slab_usable(l)) return false;
+            if (!f->slab_usable(l)) return false;
+            px += (double)v.H * v.W;
+            spx += (double)v.H * v.W * (f->streaming_ok(l) ? v.smooth : 4);
         }
     }
-    return true;
+    return px == 0 || px < std::min(kSlabBelow, kSlabBelowBase + kSlabBelowPerSmooth * (spx / px));
 }
 
 namespace {

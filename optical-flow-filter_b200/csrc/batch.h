@@ -58,10 +58,10 @@ public:
     // bands of `band` rows (<= 0: chosen per step)
     void set_tuning(long min_pixels, int band);
     static constexpr long kDefaultBeside = 200000;
-    // A phase of less than kSlabBelow pixels runs its levels by the slab kernel, in the launches
-    // that otherwise are its streaming and its tile launch, unless set_tuning or set_level_band
-    // ask for something else
-    static constexpr long kSlabBelow = 8000000;
+    // A phase of less than min(kSlabBelow, kSlabBelowBase + kSlabBelowPerSmooth * S) pixels runs its
+    // levels by the slab kernel, in the launches that otherwise are its streaming and its tile
+    // launch, unless set_tuning or set_level_band ask for something else (slab_phase)
+    static constexpr double kSlabBelow = 8e6, kSlabBelowBase = 0.5e6, kSlabBelowPerSmooth = 2.5e6;
     // levels of height x width pixels run in bands of `band` rows (<= 0: no override)
     void set_level_band(int height, int width, int band);
 

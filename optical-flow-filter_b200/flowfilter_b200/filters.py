@@ -620,9 +620,10 @@ class BatchFlowFilter:
     def setTuning(self, minPixels: int = -1, band: int = 0) -> None:
         """Top levels and levels reading the previous frame's coarse flow (phase A) below
         ``minPixels`` pixels run the tile kernel (-1: below 200000 the slab kernel), every
-        other level the streaming kernel covers runs it in bands of ``band`` rows (0: the default rule).  With the
-        defaults and no level band, a phase of fewer than 8,000,000 pixels runs all its
-        levels by the slab kernel.  Results are unchanged."""
+        other level the streaming kernel covers runs it in bands of ``band`` rows (0: the
+        default rule).  With the defaults and no level band, a phase of fewer than 0.5 + 2.5 S
+        million pixels (S: its levels' smoothing iterations, averaged over the pixels; 8 million
+        at the most) runs all its levels by the slab kernel.  Results are unchanged."""
         call("ff_batch_set_tuning", self._h, int(minPixels), int(band))
 
     @staticmethod
