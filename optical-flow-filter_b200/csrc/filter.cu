@@ -760,15 +760,22 @@ int Filter::path_of(int l, int* param) const {
         return kSlab;
     }
     if (v.tuned_path == kPerStage) return kPerStage;
-    // Untuned.  The slab kernel's rows stay in shared memory, so it holds 2048x1088 in 2-3 waves;
-    // the streaming kernel passes over HBM once at any size, but its chain of stages per row
-    // grows with S.  Measured alone (us, slab / streaming / tile), delta levels: 160x120 N 4 S 2
-    // 18.0 / 54.7 / 15.9, 320x240 20.0 / 53.2 / 19.9, 640x480 26.1 / 58.9 / 34.3, 1280x720
-    // 45.3 / 62.9 / 69.4, 2048x1088 98.3 / 89.0 / 153.2 and with S 4 120.6 / 178.2 / 223.5; top
-    // levels: 160x120 N 2 S 2 11.8 / 28.1 / 11.7, 1280x720 26.1 / 38.4 / 40.3, 2048x1088
-    // 48.8 / 50.0 / 80.8 and with S 1 43.7 / 36.7 / 69.7.
+    // Untuned.  The slab kernel's rows stay in shared memory, and it works a level in waves of one
+    // slab per SM; the streaming kernel passes over HBM once at any size, but a row's latency,
+    // which grows with S and N, takes as long on a small level.  Measured alone (us, slab / streaming
+    // / tile), delta levels: 160x120 N 4 S 2 18.0 / 54.7 / 15.9, 320x240 20.0 / 53.2 / 19.9, 640x480
+    // 26.1 / 58.9 / 34.3, 1280x720 45.3 / 62.9 / 69.4, 2048x1088 98.3 / 89.0 / 153.2 and with S 4
+    // 120.6 / 178.2 / 223.5, 3840x2160 with S 4 406 / 294; top levels: 160x120 N 2 S 2
+    // 11.8 / 28.1 / 11.7, 1280x720 26.1 / 38.4 / 40.3, 2048x1088 48.8 / 50.0 / 80.8, 3840x2160
+    // 169 / 114 / 326.  The two are level (slab / streaming 0.95 to 1.1) on delta levels at 0.9 M
+    // pixels with N 1 S 1, 1.4 M N 4 S 1, 1.5 M N 2 S 2, 1.9 M N 4 S 2, 2.2 M N 2 S 3, 2.6 M N 2 S 4
+    // and 3.2 M N 4 S 4, on top levels at 1.4, 2.3, 3.2 and 4.6 M with S 1 to 4 (with N 4 and S 3
+    // at 4 M: 2560x1440 113 / 139); on 16 M pixels streaming takes 0.5 to 0.8 of the slab's time.
     const long px = (long)v.H * v.W;
-    if (px >= kStreamMinPixels && v.smooth <= (v.delta ? 2 : 1) && fused_ok(l)) {
+    const double stream_px =
+        v.delta ? 0.2e6 + 0.55e6 * v.smooth + 0.15e6 * v.iters
+                : 0.35e6 + 1.0e6 * v.smooth + 0.07e6 * (v.iters - 1) * (v.smooth - 1);
+    if (px >= stream_px && fused_ok(l)) {
         p = band_;
         return kStream;
     }

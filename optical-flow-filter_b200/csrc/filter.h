@@ -153,8 +153,8 @@ public:
         fused_mode_ = mode;
         drop_graphs();
     }
-    // path_of's rule for untuned levels: streaming kernel from, slab kernel of delta levels from
-    static constexpr long kStreamMinPixels = 1500000, kSlabMinPixels = 76800;
+    // path_of's rule for untuned levels: slab kernel of delta levels from
+    static constexpr long kSlabMinPixels = 76800;
     // with more than 4 sub-steps or smoothing iterations: slab kernel of delta, of top levels from
     static constexpr long kSlabMinPixelsMany = 100000, kSlabMinTopMany = 30000;
     // time every candidate kernel configuration of each level on the current inputs and
