@@ -295,6 +295,14 @@ bool overlap(const Rows& a, const Rows& b, int H) { return a.begin() < b.end(H) 
 // the most sub-step pairs or smoothing iterations of one slab launch
 constexpr int kMaxFused = 8;
 
+// A single sub-step pair on rows that do not allow four pixels at a time: the slab saves one
+// launch and loads and stores pixel by pixel.  Measured (us, slab / two passes) 321x241 payload
+// 6.6 / 8.2, 641x481 9.3 / 8.2, flow 6.2 / 6.8, 1001x701 17.7 / 12.4 and 9.1 / 7.9, 2049x1089
+// 46.8 / 36.1 and 22.6 / 20.5; two pairs 0.6 to 0.85 of the passes' time, one of smoothing 0.97
+// to 1.08.  The passes from this many pixels on.
+constexpr long kSinglePixels = 500000, kSinglePixelsPayload = 200000;
+bool rows_of_caller4(bool delta, LevelArgs a) { return set_access_of_caller(delta, a) == cudaSuccess && a.vec; }
+
 template <bool DELTA, bool TAPE>
 cudaError_t launch_images(LevelArgs a, int N, int S, int images, const Tape& tape, cudaStream_t s) {
     cudaError_t e = set_access(DELTA, a);
@@ -407,6 +415,8 @@ cudaError_t launch_propagate_stage(const float* flow, size_t fp, int H, int W, i
     a.fs_in = flow, a.fs_in_pitch = fp;
     a.fs_out = out, a.fs_out_pitch = op;
     a.border = border;
+    if (N == 1 && (long)H * W >= slab::kSinglePixels && !slab::rows_of_caller4(false, a))
+        return launch_propagate(flow, fp, H, W, N, border, out, op, tmp, tp, s);
     return slab::launch_propagate_slab<false>(a, N, s);
 }
 
@@ -433,6 +443,9 @@ cudaError_t launch_propagate_payload_stage(const float* flow, size_t fp, const f
     a.io_out = os, a.io_out_pitch = osp;
     a.d_out = ov, a.d_out_pitch = ovp;
     a.border = border;
+    if (N == 1 && (long)H * W >= slab::kSinglePixelsPayload && !slab::rows_of_caller4(true, a))
+        return launch_propagate_payload(flow, fp, sc, sp, ve, vp, H, W, N, border, of, ofp, os, osp, ov, ovp, tf, tfp, ts,
+                                        tsp, tv, tvp, s);
     return slab::launch_propagate_slab<true>(a, N, s);
 }
 
