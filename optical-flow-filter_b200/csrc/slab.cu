@@ -174,13 +174,14 @@ int max_rows(bool delta, int N, int S) {
 }
 
 int sm_count() {
-    static int cache[64] = {};
+    static std::atomic<int> cache[64] = {};  // several threads may ask first
     int dev = 0;
     cudaGetDevice(&dev);
-    int& n = cache[dev & 63];
+    int n = cache[dev & 63].load(std::memory_order_relaxed);
     if (n == 0) {
         cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
         if (n <= 0) n = 148;
+        cache[dev & 63].store(n, std::memory_order_relaxed);
     }
     return n;
 }
