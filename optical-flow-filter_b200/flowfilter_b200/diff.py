@@ -641,16 +641,16 @@ _FrameStep = None
 
 def _frame_infer(flt, frame, gamma, weights, state_flat, first: bool):
     """One frame without a tape (ff_diff_frame_infer): the same outputs as _frame_forward, the
-    intermediates in a scratch buffer kept on the filter and reused every frame."""
+    intermediates in a scratch buffer kept on the filter and reused every frame by the stream that
+    made it (frames on two streams may run at the same time)."""
     d = _dt(frame)
     B = frame.shape[0]
     g = _geom(flt, B)
-    key = (d, B, frame.device)
-    cache = flt.__dict__.setdefault("_infer_scratch", {})
-    if key not in cache:
-        cache.clear()
-        cache[key] = _workspace("ff_diff_frame_infer_bytes", d, g, frame)
-    scratch = cache[key]
+    key = (d, B, frame.device, current_stream())
+    kept = flt.__dict__.get("_infer_scratch")
+    if kept is None or kept[0] != key:
+        kept = flt._infer_scratch = (key, _workspace("ff_diff_frame_infer_bytes", d, g, frame))
+    scratch = kept[1]
     new = []
     for h, w in flt.shapes:
         new += [frame.new_empty((B, h, w, 2)), frame.new_empty((B, h, w)), frame.new_empty((B, h, w, 2))]
