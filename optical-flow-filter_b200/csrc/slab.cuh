@@ -19,7 +19,7 @@
 // instruction cache (a kernel that gave every stage its own warps, rows handed over in shared
 // memory, ran out of it: 98 us where this one takes 89), and four pixels per lane give
 // independent work that covers latency with 8 warps an SM.  It issues 40% fewer instructions
-// than the tile kernel (640x480, N 4 S 2: 8.8 M against 14.6 M), whose lanes index every pixel
+// than the tile kernel (640x480, N 4 S 2: 9.0 M against 14.6 M), whose lanes index every pixel
 // of every stage.  Bound by latency within the stages: 37% of the issue slots, stalls on
 // shared-memory loads and shuffles, DRAM idle.
 // Measured alone on a delta level (us, this / streaming / tile kernel): 640x480 N 4 S 2
