@@ -176,7 +176,7 @@ struct Tape {
 template <bool DELTA>
 struct Prop {
     static constexpr int NC = DELTA ? 5 : 2;  // propagated channels: U, V [, I, DX, DY]
-    static constexpr int ROWB = planes(DELTA) * kPlane;
+    static constexpr unsigned ROWB = planes(DELTA) * kPlane;  // unsigned: a row index times it may pass 2^31, and the offsets are differences
     static constexpr int CU = 0, CV = 1;
     // channels whose upwind step the reference build fuses into one fma: all but the last
     // channel each reference kernel writes (flow .y of flowPropagate{X,Y}_k, vector .y of
@@ -457,7 +457,7 @@ struct Image<float> {
 
 template <bool DELTA, typename P>
 struct Update {
-    static constexpr int ROWB = planes(DELTA) * kPlane;
+    static constexpr unsigned ROWB = planes(DELTA) * kPlane;
     // solve2 (common.cuh) of a pixel pair; nothing but the reciprocal is per lane
     __device__ __forceinline__ static void solve_pair(float2 g, float2 ax, float2 ay, float2 yt, float2 fx, float2 fy,
                                                       float2& ox, float2& oy) {
@@ -610,7 +610,7 @@ struct Update {
 // ---------------------------------------------------------------- smoothing
 template <bool DELTA>
 struct Smooth {
-    static constexpr int ROWB = planes(DELTA) * kPlane;
+    static constexpr unsigned ROWB = planes(DELTA) * kPlane;
     struct W5 {
         float k[5];
     };
