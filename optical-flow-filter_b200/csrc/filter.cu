@@ -786,7 +786,7 @@ int Filter::path_of(int l, int* param) const {
     // and the choice is between those and the slab kernel alone.
     const bool many = (v.iters > 4 || v.smooth > 4) && v.iters + 2 * v.smooth <= 24;
     if (px >= (v.delta ? (many ? kSlabMinPixelsMany : kSlabMinPixels) : (many ? kSlabMinTopMany : 0)) && slab_ok(l))
-        return slab_pays(v.delta, v.iters, v.smooth, v.W, v.H, 1) ? kSlab : kPerStage;
+        return v.lean || slab_pays(v.delta, v.iters, v.smooth, v.W, v.H, 1) ? kSlab : kPerStage;
     if (tile_ok(l, 0)) return kTile;
     return kPerStage;
 }
@@ -1120,9 +1120,22 @@ void Filter::compute_async(cudaStream_t s) {
     bool any_first = false;
     for (const Level& v : lv_) any_first |= v.first;
     // per-stage levels get their scratch before anything is queued: a failure leaves no part of
-    // a frame behind, and there is no allocation inside a capture
-    for (int l = 0; l < L_; ++l)
-        if (!lv_[l].a0.p && path_of(l, nullptr) == kPerStage) lv_[l].alloc_scratch(s);
+    // a frame behind, and there is no allocation inside a capture.  A level that would run per
+    // stage only because it is faster does without where there is no memory for it.
+    for (int l = 0; l < L_; ++l) {
+        Level& v = lv_[l];
+        if (v.a0.p || path_of(l, nullptr) != kPerStage) continue;
+        try {
+            v.alloc_scratch(s);
+        } catch (const Error& e) {
+            v.lean = true;
+            if (e.status != FF_ERR_OUT_OF_MEMORY || path_of(l, nullptr) == kPerStage) {
+                v.lean = false;
+                throw;
+            }
+            cudaGetLastError();  // the allocation's
+        }
+    }
     if (graphs_ && !any_first && prof_count_ >= prof_cap_) {
         cudaGraphExec_t& ge = graph_exec_[cur_];
         if (!ge) {

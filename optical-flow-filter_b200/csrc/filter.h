@@ -79,6 +79,7 @@ struct Level {
     int border = 3;
     bool first = true;
     int tuned_path = -1;         // autotuned: -1 not tuned, else a Path
+    bool lean = false;           // untuned: no per-stage scratch where the slab kernel runs the level too
     int tuned_band = 0;          // streaming, slab kernel: band, slab rows; tile kernel: tile shape (0 automatic)
     Buf coarse_rows;             // int per row: coarse row its update reads (delta levels)
     void build_coarse_rows(cudaStream_t s);

@@ -59,3 +59,37 @@ def test_differentiable_forward(cuda, levels, maxflow, smooth):
         with cuda.set_grad_enabled(grad):
             flows.append(f(frames).detach())
     assert cuda.equal(flows[0], flows[1]) and cuda.equal(flows[0], flows[2])
+
+
+def test_no_memory_for_scratch(cuda):
+    """Levels that run per stage by default, because it is faster, run the slab kernel where their
+    scratch cannot be allocated; levels that are asked to run per stage fail."""
+    import flowfilter_b200 as ffb
+    from flowfilter_b200 import _lib
+
+    clip = frames_of(480, 640, 2, 1)
+    out = []
+    for fail in (False, True):
+        f = ffb.FlowFilter(480, 640)
+        f.maxflow, f.smoothIterations, f.gamma = 20.0, 8, 10.0
+        assert "per-stage" in f.tuning()
+        if fail:
+            _lib.lib().ff_debug_fail_allocation_after(2)
+        try:
+            for x in clip:
+                f.loadImage(x)
+                f.compute()
+        finally:
+            _lib.lib().ff_debug_fail_allocation_after(-1)
+        assert ("slab" if fail else "per-stage") in f.tuning()
+        out.append([f.levelState(0, k) for k in (0, 1, 2)])
+    assert same(*out)
+    f = ffb.FlowFilter(480, 640)
+    f.setFused(0)
+    f.loadImage(clip[0])
+    _lib.lib().ff_debug_fail_allocation_after(2)
+    try:
+        with pytest.raises(_lib.FFError):
+            f.compute()
+    finally:
+        _lib.lib().ff_debug_fail_allocation_after(-1)
